@@ -155,7 +155,13 @@ def run(state):
         ww = torch.empty(27, n, dtype=torch.float64, device="cuda")
         state.runs[0].calflx_static(state.arrays[0].data_ptr(), ww.data_ptr())
         return _interior_fluxes(ww, state.runs[0])
-    outs = [_array(r.params) for r in state.runs] if state.out is None else [state.out]
+    if len(state.runs) == 1:
+        out = _array(state.runs[0].params) if state.out is None else state.out
+        outs = [out]
+    else:  # the batch's results one after another in one array
+        sizes = [a.numel() // 9 for a in state.arrays]
+        out = torch.empty(sum(sizes), 9, dtype=torch.float64, device="cuda")
+        outs = out.split(sizes)
     for r, a in zip(state.runs, state.arrays):
         r.upload_prims_ptr(a.data_ptr())
     if len(state.runs) == 1:
@@ -164,7 +170,7 @@ def run(state):
         ctx.step_batch(state.runs, case["steps"])
     for r, o in zip(state.runs, outs):
         r.download_prims_ptr(o.data_ptr())
-    return _by_variable(outs)
+    return {n: out[..., v] for v, n in enumerate(NAMES)}
 
 
 def _by_variable(outs):
