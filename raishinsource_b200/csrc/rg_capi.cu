@@ -189,9 +189,9 @@ void make_tmaps(Run* R) {
     }
     // face metric (i, k, component): kMetComps components nik apart
     const double* met[3] = {d.mi, d.mc, d.mk};
-    unsigned mb[3];
-    flux_tma_met_box(mb);
     for (int dir = 1; dir <= 3 && ok; ++dir) {
+      unsigned mb[3];
+      flux_tma_met_box(dir, mb);
       const cuuint64_t dims[3] = {(cuuint64_t)d.imax, (cuuint64_t)d.kmax, (cuuint64_t)kMetComps};
       const cuuint64_t strides[2] = {(cuuint64_t)d.imax * 8, (cuuint64_t)d.nik * 8};
       const cuuint32_t bx[3] = {mb[0], mb[1], mb[2]};
@@ -1045,6 +1045,7 @@ int rg_run_admit_prep(rg_ctx* ctx, rg_prep* prep, int* run_id) {
   R->nfull = (size_t)p->imax * p->jmax * p->kmax;
   d.kmet = d.kfix;
   d.nik = (size_t)p->imax * (d.kfix ? 1 : p->kmax);
+  d.gam1 = p->gam / (p->gam - 1.0);
   d.gam = p->gam; d.cfl = p->cfl; d.dmin = p->dmin; d.pmin = p->pmin; d.pmax = p->pmax; d.tmax = p->tmax;
   std::memcpy(d.ibc, p->ibc, sizeof(d.ibc));
   d.carry_cap = kCarryCap;

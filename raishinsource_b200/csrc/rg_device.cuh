@@ -43,6 +43,80 @@ __device__ __forceinline__ float mdiv(float a, float b) { return __fdividef(a, b
 template <typename T>
 __device__ __forceinline__ T mrcp(T x) { return mdiv(T(1), x); }
 
+
+// Division, reciprocal and square root as the state functions below call
+// them, one instance per state.  IeeeMath: the operators above.  NewtonMath
+// (FP64): without the branches of a full IEEE operator, so that the
+// independent quotients of a state overlap instead of standing one behind
+// the other.  A reciprocal starts from the hardware's approximation
+// (rcp.approx.ftz.f64, about 20 bits), takes one third-order step of the
+// geometric series of 1/(1 - e), e = 1 - x y, and one Newton step on the
+// residual; a quotient corrects a y by its residual; a square root runs
+// the coupled (Goldschmidt) iteration from rsqrt.approx.ftz.f64 and corrects
+// by its residual (P. Markstein, IBM J. Res. Dev. 34, 1990; "Software
+// division and square root using Goldschmidt's algorithms", 2004).  With
+// operands whose magnitudes lie in [2^-500, 2^500) no step over- or underflows
+// and the results are the correctly rounded ones, save the reciprocal of a
+// significand of all ones, whose last bit is one too low: 1 - 2^-53, the value
+// below one that 1 - x takes for tiny x, is put right by rcp1().  note() collects the
+// operands' exponents and ok() tells whether all of them lay there.  A caller
+// that finds ok() false repeats the computation with IeeeMath (zeros,
+// subnormal, huge or non-finite operands).
+template <typename T>
+struct IeeeMath {
+  __device__ __forceinline__ T rcp(T x) { return mrcp(x); }
+  __device__ __forceinline__ T rcp1(T x) { return mrcp(x); }  // of a difference from one
+  __device__ __forceinline__ T div(T a, T b) { return mdiv(a, b); }
+  __device__ __forceinline__ T sqrt(T x) { return msqrt(x); }
+  __device__ __forceinline__ bool ok() const { return true; }
+};
+__device__ __forceinline__ double rcp_newton(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  double e = fma(-x, y, 1.0);
+  e = fma(e, e, e);
+  y = fma(y, e, y);
+  e = fma(-x, y, 1.0);
+  return fma(y, e, y);
+}
+// a / b given y = 1/b correctly rounded
+__device__ __forceinline__ double div_by_rcp(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ double sqrt_newton(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  double g = x * y, h = 0.5 * y;
+  double e = fma(-g, h, 0.5);
+  g = fma(g, e, g);
+  h = fma(h, e, h);
+  e = fma(-g, h, 0.5);
+  g = fma(g, e, g);
+  h = fma(h, e, h);
+  return fma(fma(-g, g, x), h, g);
+}
+struct NewtonMath {
+  unsigned lo = 0x7fffffffu, hi = 0u;
+  __device__ __forceinline__ void note(double x) {
+    const unsigned a = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    lo = min(lo, a);
+    hi = max(hi, a);
+  }
+  __device__ __forceinline__ double rcp(double x) { note(x); return rcp_newton(x); }
+  __device__ __forceinline__ double rcp1(double x) {
+    const double y = rcp(x);
+    return x == 0x1.fffffffffffffp-1 ? 0x1.0000000000001p0 : y;
+  }
+  __device__ __forceinline__ double div(double a, double b) { note(a); note(b); return div_by_rcp(a, b, rcp_newton(b)); }
+  __device__ __forceinline__ double sqrt(double x) { note(x); return sqrt_newton(x); }
+  __device__ __forceinline__ bool ok() const { return lo >= (1023u - 500u) << 20 && hi < (1023u + 500u) << 20; }
+};
+template <typename T>
+struct FastMath : IeeeMath<T> {};  // FP32: the approximate operators already
+template <>
+struct FastMath<double> : NewtonMath {};
+
 template <typename T>
 __device__ __forceinline__ T fmax3(T a, T b, T c) {
   T r = a;
@@ -110,6 +184,20 @@ __device__ __forceinline__ void load_met(const S* __restrict__ base, size_t nik,
   m.be1 = ld(20); m.be2 = ld(21);
   m.g3_11 = ld(22); m.g3_22 = ld(23); m.g3_33 = ld(24);
   m.idetg = ld(25);
+}
+
+// The fields a face state reads (gcov, sqrt(-g), lapse, shift, gcon3a) from a
+// staged copy of the cache's planes 0-7 and 17-24, `st` apart.
+template <typename T, typename S>
+__device__ __forceinline__ void load_met_face(const S* b, int st, MetT<T>& m) {
+  auto ld = [&](int c) -> T { return T(b[c * st]); };
+  m.g00 = ld(0); m.g01 = ld(1); m.g02 = ld(2);
+  m.g11 = ld(3); m.g12 = ld(4); m.g22 = ld(5);
+  m.g33 = ld(6);
+  m.detg = ld(8);
+  m.al = ld(9); m.ial = ld(10);
+  m.be1 = ld(11); m.be2 = ld(12);
+  m.g3_11 = ld(13); m.g3_22 = ld(14); m.g3_33 = ld(15);
 }
 
 // The derived fields of one point from its base fields: calucon's
@@ -191,15 +279,20 @@ __device__ __forceinline__ void upper_gc(const T v[4], T o[4], const MetT<T>& m)
 }
 
 // physfunc.f90:2-42
-template <typename T>
-__device__ __forceinline__ T calgfl(const T u1, const T u2, const T u3, const MetT<T>& m) {
+template <typename T, typename M>
+__device__ __forceinline__ T calgfl(const T u1, const T u2, const T u3, const MetT<T>& m, M& ma) {
   T utsq = qform3(m, u1, u2, u3);
   if (utsq < T(0)) {
     if (mabs(utsq) <= T(1.0e-10)) utsq = mabs(utsq);
     else utsq = T(1.e-10);
   }
   if (mabs(utsq) > T(5.e2)) utsq = T(5.0e2);
-  return msqrt(T(1) + utsq);
+  return ma.sqrt(T(1) + utsq);
+}
+template <typename T>
+__device__ __forceinline__ T calgfl(const T u1, const T u2, const T u3, const MetT<T>& m) {
+  IeeeMath<T> ma;
+  return calgfl(u1, u2, u3, m, ma);
 }
 
 // physfunc.f90:45-78 (alpha1, b1, b2 and 1/alpha1 from the metric cache)
@@ -217,40 +310,60 @@ template <typename T>
 struct PST {
   T ucon[4], ucov[4], bbcon[4], bbcov[4];
   T bbsq, roh, gfl, de, pr, b1, b2, b3;
+  T iu0;  // 1/u^0
 };
 using PS = PST<double>;
 
 // The state of q with a given Lorentz factor gfl (pstate below computes it
-// with calgfl; the output converter uses its own clamps).
-template <typename T>
-__device__ __forceinline__ void pstate_gfl(const T q[9], const MetT<T>& m, T gam, T gfl, PST<T>& s) {
+// with calgfl; the output converter uses its own clamps).  gam1 = gam/(gam-1).
+template <typename T, typename M>
+__device__ __forceinline__ void pstate_gfl(const T q[9], const MetT<T>& m, T gam1, T gfl, PST<T>& s, M& ma) {
   s.de = q[0];
   s.pr = q[4];
   s.b1 = q[6]; s.b2 = q[7]; s.b3 = q[8];
-  s.roh = s.de + (gam / (gam - T(1))) * s.pr;
+  s.roh = s.de + gam1 * s.pr;
   s.gfl = gfl;
   calucon(q[1], q[2], q[3], s.gfl, m, s.ucon);
   lower_g(s.ucon, s.ucov, m);
+  s.iu0 = ma.rcp(s.ucon[0]);
   // physfunc.f90:81-100
   s.bbcon[0] = s.b1 * s.ucov[1] + s.b2 * s.ucov[2] + s.b3 * s.ucov[3];
-  s.bbcon[1] = (s.b1 + s.bbcon[0] * s.ucon[1]) * mrcp(s.ucon[0]);
-  s.bbcon[2] = (s.b2 + s.bbcon[0] * s.ucon[2]) * mrcp(s.ucon[0]);
-  s.bbcon[3] = (s.b3 + s.bbcon[0] * s.ucon[3]) * mrcp(s.ucon[0]);
+  s.bbcon[1] = (s.b1 + s.bbcon[0] * s.ucon[1]) * s.iu0;
+  s.bbcon[2] = (s.b2 + s.bbcon[0] * s.ucon[2]) * s.iu0;
+  s.bbcon[3] = (s.b3 + s.bbcon[0] * s.ucon[3]) * s.iu0;
   lower_g(s.bbcon, s.bbcov, m);
   s.bbsq = s.bbcon[0] * s.bbcov[0] + s.bbcon[1] * s.bbcov[1] + s.bbcon[2] * s.bbcov[2] + s.bbcon[3] * s.bbcov[3];
 }
+template <typename T, typename M>
+__device__ __forceinline__ void pstate(const T q[9], const MetT<T>& m, T gam1, PST<T>& s, M& ma) {
+  pstate_gfl(q, m, gam1, calgfl(q[1], q[2], q[3], m, ma), s, ma);
+}
 template <typename T>
-__device__ __forceinline__ void pstate(const T q[9], const MetT<T>& m, T gam, PST<T>& s) {
-  pstate_gfl(q, m, gam, calgfl(q[1], q[2], q[3], m), s);
+__device__ __forceinline__ void pstate(const T q[9], const MetT<T>& m, T gam1, PST<T>& s) {
+  IeeeMath<T> ma;
+  pstate(q, m, gam1, s, ma);
 }
 
 // p / rho^Gamma of a state (caluu.f90:303, calflx.f90:474), computed once per state.
+template <typename T, typename M>
+__device__ __forceinline__ T ent_ratio(const PST<T>& s, T gam, int gkind, M& ma) {
+  return ma.div(s.pr, pow_gam(s.de, gam, gkind));
+}
 template <typename T>
-__device__ __forceinline__ T ent_ratio(const PST<T>& s, T gam, int gkind) { return mdiv(s.pr, pow_gam(s.de, gam, gkind)); }
+__device__ __forceinline__ T ent_ratio(const PST<T>& s, T gam, int gkind) {
+  IeeeMath<T> ma;
+  return ent_ratio(s, gam, gkind, ma);
+}
+
+// A product that is rounded by itself: the LLF flux subtracts the two states of
+// a face, and a product fused into that difference on one side only would
+// leave a rounding error where the states are equal.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 
 // caluu.f90:92-118: sqrt(-g) (rho u^t, T^t_i, T^t_t + rho u^t, s u^t, B^i).
 // delta(0,n) is the literal identity of caldelta (physfunc.f90:122-158).
-template <typename T>
+template <typename T, bool FACE = false>
 __device__ __forceinline__ void p2c(const PST<T>& s, T gam, T detg, T u[9], T sr) {
   const T a = s.roh + s.bbsq, b = s.pr + T(0.5) * s.bbsq;
   u[0] = s.de * s.ucon[0];
@@ -260,7 +373,7 @@ __device__ __forceinline__ void p2c(const PST<T>& s, T gam, T detg, T u[9], T sr
   u[5] = s.de * sr * s.ucon[0];
   u[6] = s.b1; u[7] = s.b2; u[8] = s.b3;
 #pragma unroll
-  for (int n = 0; n < 9; ++n) u[n] = detg * u[n];
+  for (int n = 0; n < 9; ++n) u[n] = FACE ? mul_rn(detg, u[n]) : detg * u[n];
 }
 template <typename T>
 __device__ __forceinline__ void p2c(const PST<T>& s, T gam, int gkind, T detg, T u[9]) {
@@ -282,34 +395,42 @@ __device__ __forceinline__ void flux(const PST<T>& s, T gam, T detg, T w[9], T s
 #pragma unroll
   for (int m = 1; m <= 3; ++m) {
     if (m == D) w[5 + m] = T(0);
-    else w[5 + m] = (ud * mrcp(s.ucon[0])) * bc[m] - (s.ucon[m] * mrcp(s.ucon[0])) * bc[D];
+    else w[5 + m] = (ud * s.iu0) * bc[m] - (s.ucon[m] * s.iu0) * bc[D];
   }
 #pragma unroll
-  for (int n = 0; n < 9; ++n) w[n] = detg * w[n];
+  for (int n = 0; n < 9; ++n) w[n] = mul_rn(detg, w[n]);
 }
 
 // calcha.f90:370-908 (icha = 2, Del Zanna et al. 2007) in direction D, using
 // the state already evaluated in PST.  cal3met (coord.f90:970-1013) gives the
 // spatial metrics: gcov3a = gcov + 0*0, gcon3a(D,D) = gcon(D,D) + (beta^D/alpha)^2.
-template <int D, typename T>
-__device__ __forceinline__ void wavespeed(const T q[9], const PST<T>& s, const MetT<T>& m, T gam, T& vfp, T& vfm) {
+template <int D, typename T, typename M>
+__device__ __forceinline__ void wavespeed(const T q[9], const PST<T>& s, const MetT<T>& m, T gam, T& vfp, T& vfm,
+                                          M& ma) {
   const T alpha1 = m.al;
   const T betad = (D == 1) ? m.be1 : (D == 2 ? m.be2 : T(0));
   const T gc3dd = (D == 1) ? m.g3_11 : (D == 2 ? m.g3_22 : m.g3_33);
-  const T vcon[4] = {T(0), q[1] * mrcp(s.gfl), q[2] * mrcp(s.gfl), q[3] * mrcp(s.gfl)};
+  const T igfl = ma.rcp(s.gfl);
+  const T vcon[4] = {T(0), q[1] * igfl, q[2] * igfl, q[3] * igfl};
   const T vsq = qform3(m, vcon[1], vcon[2], vcon[3]);
-  const T cssq = mdiv(gam * s.pr, s.roh);
-  const T vasq = s.bbsq * mrcp(s.roh + s.bbsq);
+  const T cssq = ma.div(gam * s.pr, s.roh);
+  const T vasq = s.bbsq * ma.rcp(s.roh + s.bbsq);
   const T omsq = vasq + cssq * (T(1) - vasq);
   const T f1 = vcon[D] * (T(1) - omsq);
   const T f2 = T(1) - vsq * omsq;
   const T f3 = omsq * (T(1) - vsq) * ((T(1) - vsq * omsq) * gc3dd - (T(1) - omsq) * vcon[D] * vcon[D]);
-  vfp = (f1 + msqrt(f3)) * mrcp(f2);
-  vfm = (f1 - msqrt(f3)) * mrcp(f2);
+  const T sf3 = ma.sqrt(f3), if2 = ma.rcp1(f2);
+  vfp = (f1 + sf3) * if2;
+  vfm = (f1 - sf3) * if2;
   vfp = alpha1 * vfp - betad;
   vfm = alpha1 * vfm - betad;
   if (mabs(vfp) > T(1)) vfp = T(1);
   if (mabs(vfm) > T(1)) vfm = T(-1);
+}
+template <int D, typename T>
+__device__ __forceinline__ void wavespeed(const T q[9], const PST<T>& s, const MetT<T>& m, T gam, T& vfp, T& vfm) {
+  IeeeMath<T> ma;
+  wavespeed<D>(q, s, m, gam, vfp, vfm, ma);
 }
 
 }  // namespace rg

@@ -536,7 +536,7 @@ __device__ __forceinline__ void stage_pre(const DevRun& r, int i, int j, int k, 
   double qc[9];
   load9(Pc, N, c, qc);
   PS s;
-  pstate(qc, m, gam, s);
+  pstate(qc, m, r.gam1, s);
   p2c(s, gam, r.gkind, m.detg, ucur);
   // U^n = P2C(P^n) is this stage's ucur in stage 1; stages 2 and 3 read it back
   if (STAGE == 1)
@@ -636,7 +636,7 @@ __device__ __forceinline__ void stage_pre_mixed(const DevRun& r, int i, int j, i
   double qc[9];
   load9(Pc, N, c, qc);
   PS s;
-  pstate(qc, m, gam, s);
+  pstate(qc, m, r.gam1, s);
   p2c(s, gam, r.gkind, m.detg, ucur);
   if (STAGE == 1)
 #pragma unroll
@@ -994,11 +994,6 @@ template <>
 __device__ __forceinline__ const float* met_of<3, float>(const DevRun& r) { return r.mk32; }
 
 //
-// VIEW: the stencil (and the positivity fallback) is read from a staged copy
-// of the primitives instead of P: variable v of the lane's cell at
-// Vp[v * Vn + Vc], neighbours along D Vst apart (the shared-memory box of
-// k_flux_tma).  Stores, metric and coordinates stay global.
-//
 // OUT (the per-routine rg_rec2): the lane also stores its face state, face
 // conserved variables and face flux, all nine variables (the sixth included),
 // into fo->q/u/w[side] at the face's cell index (rec.f90's uri?l/uri?r,
@@ -1008,19 +1003,15 @@ struct FaceOut {
   double* u[2];
   double* w[2];
 };
-template <int D, int IREC, typename T, typename S, bool VIEW = false, bool OUT = false>
-__device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__ P, S* __restrict__ F,
-                                          float* __restrict__ Fcopy, int icopy, int i, int j, int k, int side,
-                                          bool valid, const S* Vp = nullptr, size_t Vn = 0, size_t Vc = 0,
-                                          long long Vst = 0, const FaceOut* fo = nullptr,
-                                          const S* Mv = nullptr, int Mst = 0) {
-  const unsigned mask = __activemask();
-  const size_t N = r.N, c = r.cell(i, j, k);
-  const long long st = (D == 1) ? 1 : (D == 2 ? (long long)r.sj : (long long)r.sk);
-  const S* Pv = VIEW ? Vp : P;
-  const size_t Nv = VIEW ? Vn : N, cv = VIEW ? Vc : c;
-  const long long sv = VIEW ? Vst : st;
-  T q[9];
+// The face state of side `side` (0: left, of cell f; 1: right, of cell f+1)
+// into q: the scheme's reconstruction, then the positivity fallback.
+// PACK: the stencil's array holds the eight variables that are reconstructed
+// (all but the sixth) one after another.
+template <int D, int IREC, typename T, typename S, bool OUT, bool PACK = false>
+__device__ __forceinline__ void face_recon(const DevRun& r, const S* __restrict__ P, const S* Pv, size_t Nv, size_t cv,
+                                           long long sv, int i, int j, int k, int side, T q[9]) {
+  const size_t N = r.N;
+  auto vo = [&](int v) { return (size_t)(PACK && v > 5 ? v - 1 : v) * Nv; };
   if (IREC == 5) {
     const int f = ((D == 1) ? i : (D == 2 ? j : k)) + side;  // owner cell of this lane's state
     const double* dxs = (D == 1) ? r.dx1s : (D == 2 ? r.dx2s : r.dx3s);
@@ -1030,8 +1021,8 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
     for (int o = -2; o <= 2; ++o) dx[o + 4] = T(__ldg(dxs + f - 1 + o));
 #pragma unroll
     for (int o = -1; o <= 1; ++o) xx[o + 4] = T(__ldg(xs + f - 1 + o));
-    if (side == 0) ppm_cell<D, T, S, OUT>(Pv + cv, Nv, sv, dx, xx, T(r.gam), other, q);  // uriil(f)
-    else ppm_cell<D, T, S, OUT>(Pv + cv + sv, Nv, sv, dx, xx, T(r.gam), q, other);       // uriir(f)
+    if (side == 0) ppm_cell<D, T, S, OUT, PACK>(Pv + cv, Nv, sv, dx, xx, T(r.gam), other, q);  // uriil(f)
+    else ppm_cell<D, T, S, OUT, PACK>(Pv + cv + sv, Nv, sv, dx, xx, T(r.gam), q, other);       // uriir(f)
   } else if (IREC == 1 || IREC == 2 || IREC == 11 || IREC == 12 || IREC == 13) {
     // owner cell f of this lane's state and its coordinate's coefficients
     const int f = ((D == 1) ? i : (D == 2 ? j : k)) + side;
@@ -1046,7 +1037,7 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
 #pragma unroll
     for (int v = 0; v < 9; ++v) {
       if (v == 5 && !OUT) { q[v] = T(0); continue; }  // var 6 faces are never read downstream
-      const S* p = Pv + (size_t)v * Nv + cv + side * sv;
+      const S* p = Pv + vo(v) + cv + side * sv;
       const T u0 = T(p[0]);
       T tmp_b = T(0);
       if (cross) tmp_b = ((T(p[1]) - u0) * hpi < T(0)) ? T(-1) : T(1);
@@ -1063,15 +1054,42 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
 #pragma unroll
     for (int v = 0; v < 9; ++v) {
       if (v == 5 && !OUT) { q[v] = T(0); continue; }  // var 6 faces are never read downstream
-      const S* p = Pv + (size_t)v * Nv + cv + side * sv;
+      const S* p = Pv + vo(v) + cv + side * sv;
       q[v] = ceno_state(T(p[-2 * sv]), T(p[-sv]), T(p[0]), T(p[sv]), T(p[2 * sv]), co, side, D == 3 && side == 0);
     }
   } else if (IREC == 3) {
 #pragma unroll
     for (int v = 0; v < 9; ++v) {
       if (v == 5 && !OUT) { q[v] = T(0); continue; }  // var 6 faces are never read downstream
-      const S* p = Pv + (size_t)v * Nv + cv + side * sv;
+      const S* p = Pv + vo(v) + cv + side * sv;
       q[v] = muscl_state(T(p[-sv]), T(p[0]), T(p[sv]), side);
+    }
+  } else if (IREC == 6) {
+    // MP5 in two passes: the unlimited value and the limiter's test of every
+    // variable without a branch, so that the eight chains overlap, then the
+    // limiter of the few variables that need it (0.2 to 1.3 of a warp's eight
+    // on an evolved torus), each lane through its own list.
+    const long long sd = side ? -sv : sv;  // the right state reads its stencil mirrored
+    const T sg = side ? T(-1) : T(1);
+    const S* p0 = Pv + cv + side * sv;
+    unsigned todo = 0;
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+      if (v == 5 && !OUT) { q[v] = T(0); continue; }  // var 6 faces are never read downstream
+      const S* p = p0 + vo(v);
+      const T a2 = T(p[-2 * sd]), a1 = T(p[-sd]), u0 = T(p[0]), b1 = T(p[sd]), b2 = T(p[2 * sd]);
+      q[v] = mp5_value(a2, a1, u0, b1, b2);
+      if (!mp_monotone(q[v], a1, u0, b1)) todo |= 1u << v;
+    }
+    while (todo) {
+      const int w = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const S* p = p0 + vo(w);
+      const T a2 = T(p[-2 * sd]), a1 = T(p[-sd]), u0 = T(p[0]), b1 = T(p[sd]), b2 = T(p[2 * sd]);
+      const T lim = mp_limit_to(mp5_value(a2, a1, u0, b1, b2), a2, a1, u0, b1, b2, sg);
+#pragma unroll
+      for (int v = 0; v < 9; ++v)
+        if (v == w) q[v] = lim;
     }
   } else {
 #pragma unroll
@@ -1079,10 +1097,9 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
       if (v == 5 && !OUT) { q[v] = T(0); continue; }  // var 6 faces are never read downstream
       // owner cell f + side; the right state reads its stencil mirrored
       const long long sd = side ? -sv : sv;
-      const S* p = Pv + (size_t)v * Nv + cv + side * sv;
+      const S* p = Pv + vo(v) + cv + side * sv;
       const T a2 = T(p[-2 * sd]), a1 = T(p[-sd]), u0 = T(p[0]), b1 = T(p[sd]), b2 = T(p[2 * sd]);
-      if (IREC == 6) q[v] = mp5_state(a2, a1, u0, b1, b2, side ? T(-1) : T(1));
-      else if (IREC == 8) {
+      if (IREC == 8) {
         // mpweno5: WENO5-JS limited by MP5's bounds (rec.f90:2645-3158).  Its
         // radial right state reads uri(n,i-11,j,k) for uri(n,i-1,j,k) in beta_1
         // (rec.f90:2757); Fortran addresses it in the column-major array, so
@@ -1101,52 +1118,146 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
   }
   if ((r.guard & 1) && !(q[0] > T(0) && q[4] > T(0))) {
 #pragma unroll
-    for (int v = 0; v < 9; ++v) q[v] = T(Pv[(size_t)v * Nv + cv + side * sv]);
+    for (int v = 0; v < 9; ++v) q[v] = (PACK && v == 5) ? T(0) : T(Pv[vo(v) + cv + side * sv]);
   }
-  MetT<T> m;
-  if (VIEW && Mv) load_met<T, S, false>(Mv, (size_t)Mst, 0, m);  // the face metric staged with the stencil
-  else load_met(met_of<D, S>(r), r.nik, r.ik(i, k), m);
-  const T gam = T(r.gam);
+}
+
+// Conserved variables, flux and wave speeds of one face state.
+template <typename T>
+struct FaceSt {
   T u[9], w[9], vp, vm;
-  {
-    PST<T> s;
-    pstate(q, m, gam, s);
-    const T sr = ent_ratio(s, gam, r.gkind);
-    p2c(s, gam, m.detg, u, sr);
-    flux<D>(s, gam, m.detg, w, sr);
-    wavespeed<D>(q, s, m, gam, vp, vm);
+};
+template <int D, typename T, typename M>
+__device__ __forceinline__ void face_state_m(const T q[9], const MetT<T>& m, T gam, T gam1, int gkind, FaceSt<T>& o,
+                                             M& ma) {
+  PST<T> s;
+  pstate(q, m, gam1, s, ma);
+  const T sr = ent_ratio(s, gam, gkind, ma);
+  p2c<T, true>(s, gam, m.detg, o.u, sr);
+  flux<D>(s, gam, m.detg, o.w, sr);
+  wavespeed<D>(q, s, m, gam, o.vp, o.vm, ma);
+}
+// The same with IEEE operators, for states whose operands NewtonMath refuses.
+template <int D, typename T>
+__device__ __noinline__ void face_state_ieee(const T* q, const MetT<T>* m, T gam, T gam1, int gkind, FaceSt<T>* o) {
+  IeeeMath<T> ma;
+  face_state_m<D>(q, *m, gam, gam1, gkind, *o, ma);
+}
+template <int D, typename T>
+__device__ __forceinline__ void face_state(const T q[9], const MetT<T>& m, T gam, T gam1, int gkind, FaceSt<T>& o) {
+  FastMath<T> ma;
+  face_state_m<D>(q, m, gam, gam1, gkind, o, ma);
+  if constexpr (sizeof(T) == 8) {
+    if (!ma.ok()) {
+      T qq[9];
+#pragma unroll
+      for (int v = 0; v < 9; ++v) qq[v] = q[v];
+      MetT<T> mm = m;
+      FaceSt<T> oo;
+      face_state_ieee<D, T>(qq, &mm, gam, gam1, gkind, &oo);
+      o = oo;
+    }
   }
+}
+
+// One flux component of hll.f90:83-183 from the two states.  calcha's bounds
+// start from zero (calcha.f90:96-120: cmax = max(0, ..) >= 0 and cmin =
+// min(0, ..) <= 0, a NaN speed being passed over), so of hll's cases only
+// cmax > 0 and cmax = 0 occur.
+template <int D, typename T>
+__device__ __forceinline__ void face_bounds(T vpL, T vmL, T vpR, T vmR, T& cmax, T& c1) {
+  cmax = fmax3(T(0), vpR, vpL);
+  // (cmink uses the R-state plus speed, calcha.f90:107)
+  const T cmin = (D == 3) ? fmin3(T(0), vpR, vmL) : fmin3(T(0), vmR, vmL);
+  c1 = dmax2(mabs(cmax), mabs(cmin));
+}
+
+template <int D, int IREC, typename T, typename S, bool OUT = false>
+__device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__ P, S* __restrict__ F,
+                                          float* __restrict__ Fcopy, int icopy, int i, int j, int k, int side,
+                                          bool valid, const FaceOut* fo = nullptr) {
+  const unsigned mask = __activemask();
+  const size_t N = r.N, c = r.cell(i, j, k);
+  const long long st = (D == 1) ? 1 : (D == 2 ? (long long)r.sj : (long long)r.sk);
+  T q[9];
+  face_recon<D, IREC, T, S, OUT>(r, P, P, N, c, st, i, j, k, side, q);
+  MetT<T> m;
+  load_met(met_of<D, S>(r), r.nik, r.ik(i, k), m);
+  FaceSt<T> s;
+  face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, s);
   if constexpr (OUT) {
     if (valid) {
 #pragma unroll
       for (int v = 0; v < 9; ++v) {
         fo->q[side][(size_t)v * N + c] = double(q[v]);
-        fo->u[side][(size_t)v * N + c] = double(u[v]);
-        fo->w[side][(size_t)v * N + c] = double(w[v]);
+        fo->u[side][(size_t)v * N + c] = double(s.u[v]);
+        fo->w[side][(size_t)v * N + c] = double(s.w[v]);
       }
     }
   }
-  const T vpo = __shfl_xor_sync(mask, vp, 1), vmo = __shfl_xor_sync(mask, vm, 1);
-  const T vpL = side ? vpo : vp, vpR = side ? vp : vpo;
-  const T vmL = side ? vmo : vm, vmR = side ? vm : vmo;
-  // calcha.f90:96-120 (cmink uses the R-state plus speed, calcha.f90:107)
-  const T cmax = fmax3(T(0), vpR, vpL);
-  const T cmin = (D == 3) ? fmin3(T(0), vpR, vmL) : fmin3(T(0), vmR, vmL);
+  const T vpo = __shfl_xor_sync(mask, s.vp, 1), vmo = __shfl_xor_sync(mask, s.vm, 1);
+  T cmax, c1;
+  face_bounds<D, T>(side ? vpo : s.vp, side ? vmo : s.vm, side ? s.vp : vpo, side ? s.vm : vmo, cmax, c1);
+  const T c1s = side ? -c1 : c1;  // c1 (uR - uL) from (other - mine)
   const bool copy = Fcopy != nullptr && i <= icopy;
-  // hll.f90:83-183
+  // The even lane forms variables 0, 2, 4, 6, 8 and the odd lane 1, 3, 5, 7: a
+  // pair trades the variable each needs for the one it gives away.
+#pragma unroll
+  for (int h = 0; h < 5; ++h) {
+    const int ve = 2 * h, vo = (2 * h + 1 < 9) ? 2 * h + 1 : 8;
+    const T um = side ? s.u[vo] : s.u[ve], wm = side ? s.w[vo] : s.w[ve];
+    const T us = side ? s.u[ve] : s.u[vo], ws = side ? s.w[ve] : s.w[vo];
+    const T uo = __shfl_xor_sync(mask, us, 1), wo = __shfl_xor_sync(mask, ws, 1);
+    if (!valid || (h == 4 && side)) continue;
+    const int v = side ? vo : ve;
+    T f = (cmax > T(0)) ? T(0.5) * (wm + wo - c1s * (uo - um)) : (side ? wm : wo);
+    if (mabs(f) < T(1.0e-40)) f = T(0);
+    if ((r.guard & 2) && v == 5 + D) f = T(0);  // Toth: no flux of the normal field component
+    F[(size_t)v * N + c] = S(f);
+    if (copy) Fcopy[(size_t)v * N + c] = float(f);
+  }
+}
+
+// One thread per face, for the kernel with the stencil staged in shared
+// memory: both states in turn, so that the face's metric and indices are
+// formed once, no value crosses lanes and every lane has a flux to form.
+// Variable v of cell f at Vp[v * Vn + Vc] (PACK order), neighbours along D Vst
+// apart.  Mv: the staged face metric, planes 0-7 of the cache Mst apart and
+// then planes 17-24 (all that a face state reads), or null.  st: this thread's
+// slots, kFaceThreads apart, for the left state's conserved variables and flux
+// while the right state is formed (null: they stay in registers).
+constexpr int kFaceThreads = 128;
+template <int D, int IREC, typename T, typename S, bool STASH>
+__device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, float* __restrict__ Fcopy, int icopy,
+                                            int i, int j, int k, const S* Vp, size_t Vn, size_t Vc, long long Vst,
+                                            const S* Mv, int Mst, T* st) {
+  MetT<T> m;
+  if (Mv) load_met_face<T, S>(Mv, Mst, m);
+  else load_met(met_of<D, S>(r), r.nik, r.ik(i, k), m);
+  T q[9], vpL, vmL;
+  FaceSt<T> L, R;
+  face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 0, q);
+  face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, L);
+  vpL = L.vp;
+  vmL = L.vm;
+  if (STASH) {
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+      st[(2 * v) * kFaceThreads] = L.u[v];
+      st[(2 * v + 1) * kFaceThreads] = L.w[v];
+    }
+    asm volatile("" ::: "memory");
+  }
+  face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 1, q);
+  face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, R);
+  T cmax, c1;
+  face_bounds<D, T>(vpL, vmL, R.vp, R.vm, cmax, c1);
+  const size_t N = r.N, c = r.cell(i, j, k);
+  const bool copy = Fcopy != nullptr && i <= icopy;
 #pragma unroll
   for (int v = 0; v < 9; ++v) {
-    const T uo = __shfl_xor_sync(mask, u[v], 1), wo = __shfl_xor_sync(mask, w[v], 1);
-    if (!valid || (v & 1) != side) continue;
-    const T uL = side ? uo : u[v], uR = side ? u[v] : uo;
-    const T wL = side ? wo : w[v], wR = side ? w[v] : wo;
-    T f;
-    if (cmin > T(0)) f = wL;
-    else if (cmin <= T(0) && cmax > T(0)) {
-      const T c1 = dmax2(mabs(cmax), mabs(cmin));
-      f = T(0.5) * (wL + wR - c1 * (uR - uL));
-    } else if (cmax <= T(0)) f = wR;
-    else continue;  // NaN speeds: the reference keeps the previous ww
+    const T uL = STASH ? st[(2 * v) * kFaceThreads] : L.u[v], wL = STASH ? st[(2 * v + 1) * kFaceThreads] : L.w[v];
+    T f = (cmax > T(0)) ? T(0.5) * (wL + R.w[v] - c1 * (R.u[v] - uL)) : R.w[v];
     if (mabs(f) < T(1.0e-40)) f = T(0);
     if ((r.guard & 2) && v == 5 + D) f = T(0);  // Toth: no flux of the normal field component
     F[(size_t)v * N + c] = S(f);
@@ -1158,6 +1269,13 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
 // (registers per thread <= 65536 / (128 * blocks), in steps of 8).
 #ifndef RG_FLUX_MINB64
 #define RG_FLUX_MINB64 5
+#endif
+
+#ifndef RG_FACE_MINB64
+#define RG_FACE_MINB64 4
+#endif
+#ifndef RG_FACE_MINB32
+#define RG_FACE_MINB32 6
 #endif
 
 // Faces with radial index i in [ilo, ihi] (and the hll range in j, k) in
@@ -1215,26 +1333,29 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // three cells out), so the faces f of a block need cells f-LO .. f+1+LO.
 template <int D, typename S, int LO>
 struct TmaBox {
+  static constexpr int ROWS = kFaceThreads / 32;  // rows of 32 faces: along j (r, phi faces) or k (theta faces)
+  static constexpr int RJ = (D == 3) ? 1 : ROWS, RK = (D == 3) ? ROWS : 1;
   static constexpr int ALIGN = 16 / (int)sizeof(S);  // elements per 16 bytes
   __host__ __device__ static constexpr int up(int n) { return (n + ALIGN - 1) / ALIGN * ALIGN; }
-  // along D: 32 faces + 2 LO + 1 cells, plus the alignment slack; across: 32 faces plus slack
+  // along D: the faces + 2 LO + 1 cells, plus the alignment slack along i; across: the faces (plus slack along i)
   static constexpr int X = (D == 1) ? up(33 + 2 * LO + ALIGN - 1) : up(32 + ALIGN - 1);
-  static constexpr int Y = (D == 2) ? 2 + 2 * LO + 1 : 2;
-  static constexpr int Z = (D == 3) ? 1 + 2 * LO + 1 : 1;
-  static constexpr int PLANE = X * Y * Z;                                   // cells per variable
-  static constexpr unsigned BYTES = (unsigned)PLANE * 9u * (unsigned)sizeof(S);  // whole box
-  // FP64 runs also stage the face metric of the block's faces (MetT's
-  // components at each face's (i, k) point): MX points along i from the
-  // block's first face rounded down to 16 bytes, one k, kMetComps components,
-  // placed after the stencil box at MOFF -- where five blocks per SM still fit
-  // (at most 45 KB each; PPM's theta box leaves no room and reads the metric
-  // through L1)
+  static constexpr int Y = (D == 2) ? RJ + 2 * LO + 1 : RJ;
+  static constexpr int Z = (D == 3) ? RK + 2 * LO + 1 : RK;
+  static constexpr unsigned VBYTES = (unsigned)(X * Y * Z) * (unsigned)sizeof(S);  // one variable's box
+  static constexpr int PLANE = (int)((VBYTES + 127u) / 128u * 128u / sizeof(S));   // its pitch (boxes land on 128 B)
+  static constexpr unsigned BYTES = VBYTES * 8u;                                   // eight variables
+  // FP64 runs also stage the face metric: two boxes of 8 planes (0-7, 17-24)
+  // of MX points along i from the block's first face rounded down to 16
+  // bytes and the block's RK rows along k
+  static constexpr bool MET = sizeof(S) == 8;
   static constexpr int MX = up(32 + ALIGN - 1);
-  static constexpr unsigned MOFF = (BYTES + 127u) / 128u * 128u;
-  static constexpr unsigned MSIZE = (unsigned)MX * (unsigned)kMetComps * (unsigned)sizeof(S);
-  static constexpr bool MET = sizeof(S) == 8 && MOFF + MSIZE <= 45u * 1024u;
-  static constexpr unsigned MBYTES = MET ? MSIZE : 0u;
-  static constexpr unsigned SMEM = MET ? MOFF + MBYTES : BYTES;
+  static constexpr unsigned MOFF = 8u * (unsigned)PLANE * (unsigned)sizeof(S);
+  static constexpr unsigned MBOX = (unsigned)(MX * RK * 8) * (unsigned)sizeof(S);
+  static constexpr unsigned MBYTES = MET ? 2u * MBOX : 0u;
+  // and keep the left states' 18 values of each thread
+  static constexpr bool STASH = sizeof(S) == 8;
+  static constexpr unsigned SOFF = MOFF + (MBYTES + 127u) / 128u * 128u;
+  static constexpr unsigned SMEM = SOFF + (STASH ? 18u * kFaceThreads * (unsigned)sizeof(S) : 0u);
 };
 template <int IREC>
 __host__ __device__ constexpr int tma_lo() { return IREC == 5 ? 3 : 2; }
@@ -1262,16 +1383,15 @@ __device__ __forceinline__ bool tma_wait(unsigned bar, const unsigned long long*
 }
 
 template <int D, int IREC, typename T, typename S>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? RG_FLUX_MINB64 : 8)
+__global__ void __launch_bounds__(kFaceThreads, sizeof(T) == 8 ? RG_FACE_MINB64 : RG_FACE_MINB32)
     k_flux_tma(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmm, DevRun r,
                S* __restrict__ F, float* __restrict__ Fcopy, int icopy, int ilo, int ihi) {
   extern __shared__ __align__(128) unsigned char box_raw[];
   __shared__ __align__(8) unsigned long long bar;
-  if (!r.scal->active) return;
   using B = TmaBox<D, S, tma_lo<IREC>()>;
   S* box = reinterpret_cast<S*>(box_raw);
   const int nm0 = r.nm0;
-  const int fi0 = ilo + (int)blockIdx.x * 32, fj0 = nm0 + 2 * (int)blockIdx.y, fk0 = nm0 + (int)blockIdx.z;
+  const int fi0 = ilo + (int)blockIdx.x * 32, fj0 = nm0 + B::RJ * (int)blockIdx.y, fk0 = nm0 + B::RK * (int)blockIdx.z;
   // 0-based origin of the box: the first stencil cell along D, the block's
   // first face elsewhere; along i rounded down to a 16-byte boundary
   constexpr int LO = tma_lo<IREC>();
@@ -1281,39 +1401,44 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? RG_FLUX_MINB64 : 8)
   const int mx0 = (fi0 - 1) & ~(B::ALIGN - 1);  // first metric point (0-based i) of the metric box
   const unsigned bar_a = (unsigned)__cvta_generic_to_shared(&bar);
   const unsigned box_a = (unsigned)__cvta_generic_to_shared(box_raw);
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  const int tid = threadIdx.x + 32 * threadIdx.y;
+  // the copies start before the run's state is known: a finished run lets them land and returns
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_a), "r"(B::BYTES + B::MBYTES)
                  : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-        "%5}], [%6];" ::"r"(box_a),
-        "l"(reinterpret_cast<unsigned long long>(&tm)), "r"(x0), "r"(y0), "r"(z0), "r"(0), "r"(bar_a)
-        : "memory");
-    if (B::MET)
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
       asm volatile(
-          "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
-          "%4}], [%5];" ::"r"(box_a + B::MOFF),
-          "l"(reinterpret_cast<unsigned long long>(&tmm)), "r"(mx0), "r"(fk0 - 1), "r"(0), "r"(bar_a)
+          "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
+          "%5}], [%6];" ::"r"(box_a + (unsigned)(b * B::PLANE) * (unsigned)sizeof(S)),
+          "l"(reinterpret_cast<unsigned long long>(&tm)), "r"(x0), "r"(y0), "r"(z0), "r"(b < 5 ? b : b + 1), "r"(bar_a)
           : "memory");
+    if (B::MET)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+        asm volatile(
+            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+            "%4}], [%5];" ::"r"(box_a + B::MOFF + b * B::MBOX),
+            "l"(reinterpret_cast<unsigned long long>(&tmm)), "r"(mx0), "r"(fk0 - 1), "r"(b ? 17 : 0), "r"(bar_a)
+            : "memory");
   }
+  const int active = r.scal->active;
   __syncthreads();
   if (!tma_wait(bar_a, r.cnt + C_TMAWAIT)) {
     if (tid == 0) atomicAdd(r.cnt + C_TMAWAIT, 1ull);
-    tma_wait(bar_a, nullptr);  // the copy in flight writes this block's shared memory: give it one more bounded wait
+    tma_wait(bar_a, nullptr);  // the copies in flight write this block's shared memory: one more bounded wait
     return;
   }
-  const int side = threadIdx.x & 1;
-  const int i0 = fi0 + (int)(threadIdx.x >> 1), j0 = fj0 + (int)threadIdx.y;
-  const bool valid = i0 <= ihi && j0 <= r.jmax - nm0 && fk0 <= r.kmax - nm0;
-  const int i = min(i0, ihi), j = min(j0, r.jmax - nm0), k = min(fk0, r.kmax - nm0);
+  const int ty = (int)threadIdx.y;
+  const int i = fi0 + (int)threadIdx.x, j = fj0 + (D == 3 ? 0 : ty), k = fk0 + (D == 3 ? ty : 0);
+  if (!active || i > ihi || j > r.jmax - nm0 || k > r.kmax - nm0) return;
   const size_t vc = (size_t)((i - 1 - x0) + B::X * ((j - 1 - y0) + B::Y * (k - 1 - z0)));
   const long long vst = (D == 1) ? 1 : (D == 2 ? B::X : B::X * B::Y);
-  const S* met = B::MET ? reinterpret_cast<const S*>(box_raw + B::MOFF) + (i - 1 - mx0) : nullptr;
-  face_lane<D, IREC, T, S, true>(r, nullptr, F, Fcopy, icopy, i, j, k, side, valid, box, B::PLANE, vc, vst, nullptr,
-                                 met, B::MX);
+  const S* met = B::MET ? reinterpret_cast<const S*>(box_raw + B::MOFF) + (i - 1 - mx0) + B::MX * (k - fk0) : nullptr;
+  T* st = B::STASH ? reinterpret_cast<T*>(box_raw + B::SOFF) + tid : nullptr;
+  face_thread<D, IREC, T, S, B::STASH>(r, F, Fcopy, icopy, i, j, k, box, B::PLANE, vc, vst, met, B::MX * B::RK, st);
 }
 
 // ------------------------------------------------ TMA-staged stage update
@@ -1568,7 +1693,7 @@ __global__ void __launch_bounds__(128, RG_FLUX_MINB64) k_rec2(DevRun r, const do
   const int k0 = kidx(r, nm0, blockIdx);
   const bool valid = i0 <= ihi && j0 <= r.jmax - nm0 && k0 <= r.kmax - nm0;
   const int i = min(i0, ihi), j = min(j0, r.jmax - nm0), k = min(k0, r.kmax - nm0);
-  face_lane<D, IREC, double, double, false, true>(r, P, F, nullptr, 0, i, j, k, side, valid, nullptr, 0, 0, 0, &fo);
+  face_lane<D, IREC, double, double, true>(r, P, F, nullptr, 0, i, j, k, side, valid, &fo);
 }
 
 // calcha (calcha.f90:2-126, with cmink built from the R state's plus speed,
@@ -1590,12 +1715,12 @@ __global__ void __launch_bounds__(128) k_calcha(DevRun r, const double* __restri
   load9(QR, N, c, qR);
   {
     PS s;
-    pstate(qL, m, r.gam, s);
+    pstate(qL, m, r.gam1, s);
     wavespeed<D>(qL, s, m, r.gam, vpL, vmL);
   }
   {
     PS s;
-    pstate(qR, m, r.gam, s);
+    pstate(qR, m, r.gam1, s);
     wavespeed<D>(qR, s, m, r.gam, vpR, vmR);
   }
   cmax[c] = fmax3(0.0, vpR, vpL);
@@ -2016,7 +2141,7 @@ __device__ __forceinline__ void floor_body(const DevRun& r, double* __restrict__
     for (int v = 0; v < 9; ++v) lim[v] = q[v];
     lim[1] = vel[1] * gfl; lim[2] = vel[2] * gfl; lim[3] = vel[3] * gfl;
     PS s;
-    pstate(lim, m, gam, s);
+    pstate(lim, m, r.gam1, s);
     const double bbsq = s.bbsq;
     gfl = s.gfl;
     const double bcon[4] = {0.0, q[6], q[7], q[8]};
@@ -2027,7 +2152,7 @@ __device__ __forceinline__ void floor_body(const DevRun& r, double* __restrict__
     bool capped = false;
     for (int cnt = 0;; ++cnt) {
       if (cnt >= 100000) { capped = true; break; }
-      const double roh = de + (gam / (gam - 1.0)) * pr;
+      const double roh = de + r.gam1 * pr;
       const double t1a = roh * gfl * gfl - pr;
       const double t1b = fabs(f005 * bsq);
       if (t1a <= t1b) { de = f105 * de; pr = f105 * pr; continue; }
@@ -2089,7 +2214,7 @@ __device__ __forceinline__ void cfl_body(const DevRun& r, const double* __restri
     Met m;
     load_met(r.mc, r.nik, r.ik(i, k), m);
     PS s;
-    pstate(q, m, r.gam, s);
+    pstate(q, m, r.gam1, s);
     double vp1, vm1, vp2, vm2, vp3, vm3;
     wavespeed<1>(q, s, m, r.gam, vp1, vm1);
     wavespeed<2>(q, s, m, r.gam, vp2, vm2);
@@ -2290,7 +2415,7 @@ __global__ void __launch_bounds__(128) k_p2c(DevRun r, const double* __restrict_
   Met m;
   load_met(r.mc, r.nik, r.ik(i, k), m);
   PS s;
-  pstate(q, m, r.gam, s);
+  pstate(q, m, r.gam1, s);
   p2c(s, r.gam, r.gkind, m.detg, u);
 #pragma unroll
   for (int v = 0; v < 9; ++v) U[(size_t)v * N + c] = u[v];
@@ -2309,7 +2434,7 @@ __global__ void __launch_bounds__(128) k_calsf(DevRun r, const double* __restric
   Met m;
   load_met(r.mc, r.nik, q, m);
   PS s;
-  pstate(p, m, r.gam, s);
+  pstate(p, m, r.gam1, s);
   double sf[4];
   geom_source(r, s, q, m.detg, sf);
 #pragma unroll
@@ -2343,7 +2468,8 @@ __device__ void derived_cell(const DevRun& r, double akm, const double qin[9], c
   for (int v = 6; v < 9; ++v)
     if (fabs(q[v]) < 1.e-20) q[v] = 0.0;
   PS s;
-  pstate_gfl(q, m, r.gam, calgfl_conv(q[1], q[2], q[3], m), s);
+  IeeeMath<double> ma;
+  pstate_gfl(q, m, r.gam1, calgfl_conv(q[1], q[2], q[3], m), s, ma);
   out[2] = s.bbsq;
   out[3] = -(s.roh / s.de) * s.ucov[0];
   const double rbh1 = 1. + sqrt(1. - akm * akm);
@@ -2602,20 +2728,24 @@ template <int IREC, typename T, typename S>
 static void launch_flux_tma_irec(const DevRun& r, int dir, const CUtensorMap& tm, const CUtensorMap& tmm, S* F,
                                  float* Fcopy, int icopy, int ilo, int ihi, dim3 g, dim3 b, cudaStream_t s) {
   constexpr int LO = tma_lo<IREC>();
-  if (dir == 1)
-    k_flux_tma<1, IREC, T, S><<<g, b, TmaBox<1, S, LO>::SMEM, s>>>(tm, tmm, r, F, Fcopy, icopy, ilo, ihi);
-  else if (dir == 2)
-    k_flux_tma<2, IREC, T, S><<<g, b, TmaBox<2, S, LO>::SMEM, s>>>(tm, tmm, r, F, Fcopy, icopy, ilo, ihi);
-  else
-    k_flux_tma<3, IREC, T, S><<<g, b, TmaBox<3, S, LO>::SMEM, s>>>(tm, tmm, r, F, Fcopy, icopy, ilo, ihi);
+  auto go = [&](auto kern, unsigned smem) {
+    // above the default 48 KB the size has to be allowed on the current device (set again on each call: it is
+    // per device and costs about a microsecond)
+    if (smem > 48u * 1024u) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<g, b, smem, s>>>(tm, tmm, r, F, Fcopy, icopy, ilo, ihi);
+  };
+  if (dir == 1) go(k_flux_tma<1, IREC, T, S>, TmaBox<1, S, LO>::SMEM);
+  else if (dir == 2) go(k_flux_tma<2, IREC, T, S>, TmaBox<2, S, LO>::SMEM);
+  else go(k_flux_tma<3, IREC, T, S>, TmaBox<3, S, LO>::SMEM);
 }
 template <typename T, typename S>
 static void launch_flux_tma_t(const DevRun& r, int dir, const CUtensorMap& tm, const CUtensorMap& tmm, S* F,
                               float* Fcopy, int icopy, int ilo, int ihi, cudaStream_t s) {
   if (ihi < ilo) return;
   const int n = ihi - ilo + 1, m = r.jmax - 2 * r.nm0 + 1, l = r.kmax - 2 * r.nm0 + 1;
-  const dim3 b(64, 2, 1);
-  const dim3 g((unsigned)((n + 31) / 32), (unsigned)((m + 1) / 2), (unsigned)l);
+  constexpr unsigned R = kFaceThreads / 32;
+  const dim3 b(32, R, 1);
+  const dim3 g((unsigned)((n + 31) / 32), dir == 3 ? (unsigned)m : (m + R - 1) / R, dir == 3 ? (l + R - 1) / R : (unsigned)l);
   switch (r.irec) {
     case 5: launch_flux_tma_irec<5, T, S>(r, dir, tm, tmm, F, Fcopy, icopy, ilo, ihi, g, b, s); break;
     case 7: launch_flux_tma_irec<7, T, S>(r, dir, tm, tmm, F, Fcopy, icopy, ilo, ihi, g, b, s); break;
@@ -2644,11 +2774,11 @@ cudaError_t launch_flux_tma(const DevRun& r, int dir, const void* tmap64, const 
   return cudaGetLastError();
 }
 
-// Box of the face-metric tensor map (i, k, component) of the staged FP64 face kernel.
-void flux_tma_met_box(unsigned box[3]) {
+// Box of the face-metric tensor map (i, k, component) of the staged FP64 face kernel of direction dir.
+void flux_tma_met_box(int dir, unsigned box[3]) {
   box[0] = TmaBox<1, double, 2>::MX;
-  box[1] = 1;
-  box[2] = kMetComps;
+  box[1] = dir == 3 ? TmaBox<3, double, 2>::RK : 1;
+  box[2] = 8;
 }
 
 template <typename S, int LO>
@@ -2656,7 +2786,7 @@ static void tma_box_of(int dir, unsigned box[4]) {
   box[0] = dir == 1 ? TmaBox<1, S, LO>::X : (dir == 2 ? TmaBox<2, S, LO>::X : TmaBox<3, S, LO>::X);
   box[1] = dir == 1 ? TmaBox<1, S, LO>::Y : (dir == 2 ? TmaBox<2, S, LO>::Y : TmaBox<3, S, LO>::Y);
   box[2] = dir == 1 ? TmaBox<1, S, LO>::Z : (dir == 2 ? TmaBox<2, S, LO>::Z : TmaBox<3, S, LO>::Z);
-  box[3] = 9;
+  box[3] = 1;
 }
 void flux_tma_box(int dir, int elem_bytes, int irec, unsigned box[4]) {
   const bool ppm = (irec == 5);

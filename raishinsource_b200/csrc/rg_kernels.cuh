@@ -36,7 +36,7 @@ void flux_tma_box(int dir, int elem_bytes, int irec, unsigned box[4]);
 // flux_tma_met_box), staged with the stencil
 cudaError_t launch_flux_tma(const DevRun& r, int dir, const void* tmap64, const void* tmap32, const void* tmapm,
                             double* F, cudaStream_t s);
-void flux_tma_met_box(unsigned box[3]);
+void flux_tma_met_box(int dir, unsigned box[3]);
 // P: the stage's primitives (upflct's upwinding reads their velocities)
 cudaError_t launch_ct(const DevRun& r, const double* P, const double* F1, const double* F2, const double* F3,
                       double* CT, cudaStream_t s);

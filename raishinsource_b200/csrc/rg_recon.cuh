@@ -45,12 +45,19 @@ __device__ __forceinline__ T dm4(T ww, T xx, T yy, T zz) {
 // (u0 - 2 u+1) + u+2, for both states, and a sum taken in the mirrored order
 // can round differently; the right state therefore picks its operands so
 // that each difference is summed as the reference sums it.
+//
+// mp_monotone: the test that lets the unlimited value ul1 stand
+// (rec.f90:2092); mp_limit_to: the limited value otherwise.
 template <typename T>
-__device__ __forceinline__ T mp_limit(T ul1, T a2, T a1, T u0, T b1, T b2, T sg) {
-  const T tmp2 = T(4.0) / T(3.0), alpha = T(4.0), eps1 = T(1.0e-10);
+__device__ __forceinline__ bool mp_monotone(T ul1, T a1, T u0, T b1) {
+  const T alpha = T(4.0), eps1 = T(1.0e-10);
   const T ulmp = u0 + dmm(b1 - u0, alpha * (u0 - a1));
   const T t = (ul1 - u0) * (ul1 - ulmp);
-  if (t <= eps1) return ul1;
+  return t <= eps1;
+}
+template <typename T>
+__device__ __forceinline__ T mp_limit_to(T ul1, T a2, T a1, T u0, T b1, T b2, T sg) {
+  const T tmp2 = T(4.0) / T(3.0), alpha = T(4.0);
   const bool right = sg < T(0);
   // left: dim1 = (a2 - 2 a1) + u0, di1 = (a1 - 2 u0) + b1, dip1 = (u0 - 2 b1) + b2;
   // right (a = u+, b = u-): dim1 = (u0 - 2 a1) + a2, di1 = (b1 - 2 u0) + a1, dip1 = (b2 - 2 b1) + u0
@@ -69,10 +76,20 @@ __device__ __forceinline__ T mp_limit(T ul1, T a2, T a1, T u0, T b1, T b2, T sg)
   return ul1 + dmm(umin - ul1, umax - ul1);
 }
 template <typename T>
-__device__ __forceinline__ T mp5_state(T a2, T a1, T u0, T b1, T b2, T sg) {
+__device__ __forceinline__ T mp_limit(T ul1, T a2, T a1, T u0, T b1, T b2, T sg) {
+  return mp_monotone(ul1, a1, u0, b1) ? ul1 : mp_limit_to(ul1, a2, a1, u0, b1, b2, sg);
+}
+// The unlimited value.  Its roundings are spelled out (in the uncontracted
+// build they are the reference's), so that every pass and kernel that forms it
+// gets the same bits whatever it goes on to do with it.
+template <typename T>
+__device__ __forceinline__ T mp5_value(T a2, T a1, T u0, T b1, T b2) {
   const T tmp1 = T(1.0) / T(60.0);
-  const T ul1 = tmp1 * (T(2.) * a2 - T(13.) * a1 + T(47.) * u0 + T(27.) * b1 - T(3.) * b2);
-  return mp_limit(ul1, a2, a1, u0, b1, b2, sg);
+#ifdef RG_EXACT_ARITH
+  return tmp1 * (T(2.) * a2 - T(13.) * a1 + T(47.) * u0 + T(27.) * b1 - T(3.) * b2);
+#else
+  return mul_rn(tmp1, fma(T(-3.), b2, fma(T(27.), b1, fma(T(47.), u0, fma(T(2.), a2, -mul_rn(T(13.), a1))))));
+#endif
 }
 
 // rec.f90:2373-2643 (WENO5-JS); the left state at +1/2 takes
@@ -304,10 +321,11 @@ __device__ __forceinline__ T ppm_face(T u0, T u1, T dma0, T dma1, T dxm, T dx0, 
 // stride st along direction D; dx[o+4], x[o+4] are the shifted spacing and
 // centre at offset o from the cell.  gam enters the contact test (rec.f90:1623).
 // ALL: also the sixth variable (the per-routine rec2 outputs every face state).
-template <int D, typename T, typename S, bool ALL = false>
+// PACK: p holds the eight other variables one after another.
+template <int D, typename T, typename S, bool ALL = false, bool PACK = false>
 __device__ void ppm_cell(const S* __restrict__ p, size_t N, long long st, const T dx[9], const T x[9], T gam,
                          T L[9], T R[9]) {
-  auto U = [&](int v, int o) { return T(p[(size_t)v * N + o * st]); };
+  auto U = [&](int v, int o) { return T(p[(size_t)(PACK && v > 5 ? v - 1 : v) * N + o * st]); };
   auto DX = [&](int o) { return dx[o + 4]; };
   // detect (rec.f90:1479-1686): contact steepening factor eta on density
   T eta;

@@ -71,6 +71,7 @@ struct DevRun {
   size_t N;              // stored cells (imax * jpl * kpl)
   size_t nik;            // (i,k) points of the metric caches (imax for a theta slab)
   double gam, cfl, dmin, pmin, pmax, tmax;
+  double gam1;           // gam/(gam-1)
   const double* mc;      // metric at cell centres (also the phi faces)
   const double* mi;      // metric at the r faces x1a(i)
   const double* mk;      // metric at the theta faces x3a(k)
