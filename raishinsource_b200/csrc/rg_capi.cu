@@ -400,6 +400,36 @@ std::vector<double> shifted(const std::vector<double>& v, int n) {
   return o;
 }
 
+// PPM's coefficients of one axis (PpmCoef in rg_recon.cuh) for the cells whose
+// stencil of spacings lies inside it, in FP64 as the reference writes them
+// (rec.f90:1346-1468, 1479-1686); dx is rec2's shifted spacing, x the centres.
+std::vector<double> ppm_coefs(const Axis& ax, int n) {
+  const std::vector<double> sh = shifted(ax.dxb, n);
+  auto dx = [&](int m) { return sh[m - 1]; };
+  std::vector<double> o(kPpmPlanes * (size_t)n, 0.0);
+  for (int m = 2; m <= n - 2; ++m) {
+    double* q = o.data() + m - 1;
+    const double a = dx(m - 1), b = dx(m), c = dx(m + 1), d = dx(m + 2);
+    q[0] = b / (a + b + c);
+    q[n] = (2.0 * a + b) / (c + b);
+    q[2 * n] = (b + 2.0 * c) / (a + b);
+    q[3 * n] = b / (b + c);
+    const double t3a = 1.0 / (a + b + c + d);
+    const double t3b = (2.0 * c * b) / (b + c);
+    const double t3c = ((a + b) / (2.0 * b + c)) - ((d + c) / (2.0 * c + b));
+    q[4 * n] = t3a * t3b * t3c;
+    q[5 * n] = t3a * b * ((a + b) / (2.0 * b + c));
+    q[6 * n] = t3a * c * ((c + d) / (b + 2.0 * c));
+    q[7 * n] = 1.0 / (a + b + c);
+    q[8 * n] = c + b;
+    q[9 * n] = 1.0 / (c + b);
+    q[10 * n] = ax.x[m + 1] - ax.x[m - 1];
+    const double e = ax.x[m] - ax.x[m - 1], f = ax.x[m + 1] - ax.x[m];
+    q[11 * n] = e * e * e + f * f * f;
+  }
+  return o;
+}
+
 // The per-routine entry points compute in FP64 on the reference's full
 // array layout, whatever the run's precision and slab directions.
 DevRun full_view(const Run* R) {
@@ -1120,14 +1150,12 @@ int rg_run_admit_prep(rg_ctx* ctx, rg_prep* prep, int* run_id) {
   if ((rc = upload(zero_based(G.ax[0].dxb, p->imax), &d.dx1b, R, s))) return bail(rc);
   if ((rc = upload(zero_based(G.ax[1].dxb, p->jmax), &d.dx2b, R, s))) return bail(rc);
   if ((rc = upload(zero_based(G.ax[2].dxb, p->kmax), &d.dx3b, R, s))) return bail(rc);
-  if ((rc = upload(zero_based(G.ax[1].x, p->jmax), &d.x2, R, s))) return bail(rc);
-  if ((rc = upload(zero_based(G.ax[2].x, p->kmax), &d.x3, R, s))) return bail(rc);
-  if ((rc = upload(shifted(G.ax[0].dxb, p->imax), &d.dx1s, R, s))) return bail(rc);
-  if ((rc = upload(shifted(G.ax[1].dxb, p->jmax), &d.dx2s, R, s))) return bail(rc);
-  if ((rc = upload(shifted(G.ax[2].dxb, p->kmax), &d.dx3s, R, s))) return bail(rc);
   const int ext[3] = {p->imax, p->jmax, p->kmax};
   for (int a = 0; a < 3; ++a)
     if ((rc = upload(limiter_coefs(G.ax[a], ext[a], p->metric == 403, p->irec), &d.lim[a], R, s))) return bail(rc);
+  if (p->irec == 5)
+    for (int a = 0; a < 3; ++a)
+      if ((rc = upload(ppm_coefs(G.ax[a], ext[a]), &d.ppm[a], R, s))) return bail(rc);
   // the caches and floor tables are this run's own allocations: fill their derived parts
   if (launch_geom_derive(d, const_cast<double*>(d.mc), const_cast<double*>(d.mi), const_cast<double*>(d.mk),
                          const_cast<double*>(d.fl_de), const_cast<double*>(d.fl_pr), s) != cudaSuccess)

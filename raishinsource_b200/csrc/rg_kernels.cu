@@ -1003,6 +1003,16 @@ struct FaceOut {
   double* u[2];
   double* w[2];
 };
+// The positivity fallback (guard bit 1): a face state with rho <= 0 or p <= 0
+// takes its owner cell's primitives (at p, variables N apart; PACK as below).
+template <typename T, typename S, bool PACK>
+__device__ __forceinline__ void face_positive(const DevRun& r, const S* p, size_t N, T q[9]) {
+  if ((r.guard & 1) && !(q[0] > T(0) && q[4] > T(0))) {
+#pragma unroll
+    for (int v = 0; v < 9; ++v) q[v] = (PACK && v == 5) ? T(0) : T(p[(size_t)(PACK && v > 5 ? v - 1 : v) * N]);
+  }
+}
+
 // The face state of side `side` (0: left, of cell f; 1: right, of cell f+1)
 // into q: the scheme's reconstruction, then the positivity fallback.
 // PACK: the stencil's array holds the eight variables that are reconstructed
@@ -1014,15 +1024,8 @@ __device__ __forceinline__ void face_recon(const DevRun& r, const S* __restrict_
   auto vo = [&](int v) { return (size_t)(PACK && v > 5 ? v - 1 : v) * Nv; };
   if (IREC == 5) {
     const int f = ((D == 1) ? i : (D == 2 ? j : k)) + side;  // owner cell of this lane's state
-    const double* dxs = (D == 1) ? r.dx1s : (D == 2 ? r.dx2s : r.dx3s);
-    const double* xs = (D == 1) ? r.x1 : (D == 2 ? r.x2 : r.x3);
-    T dx[9], xx[9], other[9];
-#pragma unroll
-    for (int o = -2; o <= 2; ++o) dx[o + 4] = T(__ldg(dxs + f - 1 + o));
-#pragma unroll
-    for (int o = -1; o <= 1; ++o) xx[o + 4] = T(__ldg(xs + f - 1 + o));
-    if (side == 0) ppm_cell<D, T, S, OUT, PACK>(Pv + cv, Nv, sv, dx, xx, T(r.gam), other, q);  // uriil(f)
-    else ppm_cell<D, T, S, OUT, PACK>(Pv + cv + sv, Nv, sv, dx, xx, T(r.gam), q, other);       // uriir(f)
+    const int n = (D == 1) ? r.imax : (D == 2 ? r.jmax : r.kmax);
+    ppm_cell<D, T, S, OUT>(Pv + cv + side * sv, Nv, sv, r.ppm[D - 1] + f - 1, n, T(r.gam), side, q);
   } else if (IREC == 1 || IREC == 2 || IREC == 11 || IREC == 12 || IREC == 13) {
     // owner cell f of this lane's state and its coordinate's coefficients
     const int f = ((D == 1) ? i : (D == 2 ? j : k)) + side;
@@ -1116,10 +1119,7 @@ __device__ __forceinline__ void face_recon(const DevRun& r, const S* __restrict_
       else q[v] = weno5_state(a2, a1, u0, b1, b2);
     }
   }
-  if ((r.guard & 1) && !(q[0] > T(0) && q[4] > T(0))) {
-#pragma unroll
-    for (int v = 0; v < 9; ++v) q[v] = (PACK && v == 5) ? T(0) : T(Pv[vo(v) + cv + side * sv]);
-  }
+  face_positive<T, S, PACK>(r, Pv + cv + side * sv, Nv, q);
 }
 
 // Conserved variables, flux and wave speeds of one face state.
@@ -1234,10 +1234,41 @@ __device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, 
   MetT<T> m;
   if (Mv) load_met_face<T, S>(Mv, Mst, m);
   else load_met(met_of<D, S>(r), r.nik, r.ik(i, k), m);
-  T q[9], vpL, vmL;
+  T q[9], qR[9], vpL, vmL;
   FaceSt<T> L, R;
-  face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 0, q);
+  if constexpr (IREC == 5) {
+    const int f = (D == 1) ? i : (D == 2 ? j : k), n = (D == 1) ? r.imax : (D == 2 ? r.jmax : r.kmax);
+    const double* pc = r.ppm[D - 1] + f - 1;
+    q[5] = qR[5] = T(0);
+    if constexpr (STASH) {
+      // through the slots: the left state in 0-8, the right one in 9-17, which
+      // are read back before the left state's values take their place
+      ppm_face_pair<D, T, S, true, true>(Vp + Vc, Vn, Vst, pc, n, T(r.gam), [&](int v, T a, T b) {
+        st[v * kFaceThreads] = a;
+        st[(9 + v) * kFaceThreads] = b;
+      });
+      asm volatile("" ::: "memory");
+#pragma unroll
+      for (int v = 0; v < 9; ++v)
+        if (v != 5) q[v] = st[v * kFaceThreads];
+    } else {
+      ppm_face_pair<D, T, S, true, false>(Vp + Vc, Vn, Vst, pc, n, T(r.gam), [&](int v, T a, T b) {
+        q[v] = a;
+        qR[v] = b;
+      });
+    }
+    face_positive<T, S, true>(r, Vp + Vc, Vn, q);
+  } else {
+    face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 0, q);
+  }
   face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, L);
+  if (IREC == 5) {
+    if (STASH)
+#pragma unroll
+      for (int v = 0; v < 9; ++v)
+        if (v != 5) qR[v] = st[(9 + v) * kFaceThreads];
+    face_positive<T, S, true>(r, Vp + Vc + Vst, Vn, qR);
+  }
   vpL = L.vp;
   vmL = L.vm;
   if (STASH) {
@@ -1248,7 +1279,12 @@ __device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, 
     }
     asm volatile("" ::: "memory");
   }
-  face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 1, q);
+  if constexpr (IREC == 5) {
+#pragma unroll
+    for (int v = 0; v < 9; ++v) q[v] = qR[v];
+  } else {
+    face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 1, q);
+  }
   face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, R);
   T cmax, c1;
   face_bounds<D, T>(vpL, vmL, R.vp, R.vm, cmax, c1);

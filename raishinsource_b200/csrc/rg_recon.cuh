@@ -288,16 +288,31 @@ __device__ __forceinline__ T muscl_state(T um, T u0, T up, int side) {
 // (uriil(c)).  dx is rec2's shifted dx?b (dummy dx?b(m) = actual dx?b(m-1),
 // rec.f90:58), x the cell centres (contact detection).
 
+// The coefficients of the spacings are the run's (PpmCoef planes of
+// DevRun::ppm, rg_capi.cu): each is the reference's expression in its order,
+// evaluated once per index instead of once per cell, variable and face (about
+// 40 divisions a cell and variable), so the values are the same.
+// Planes at 0-based index m-1, with dx(m) the shifted spacing:
+enum PpmCoef {
+  PC_A = 0,  // dx(m) / (dx(m-1) + dx(m) + dx(m+1))
+  PC_B,      // (2 dx(m-1) + dx(m)) / (dx(m+1) + dx(m))
+  PC_C,      // (dx(m) + 2 dx(m+1)) / (dx(m-1) + dx(m))
+  PC_T2,     // interface m+1/2: dx(m) / (dx(m) + dx(m+1))
+  PC_T3, PC_T4, PC_T5,
+  PC_D,      // contact: 1 / (dx(m-1) + dx(m) + dx(m+1))
+  PC_S, PC_RS,   // dx(m) + dx(m+1) and its reciprocal
+  PC_X,      // x(m+1) - x(m-1)
+  PC_X3,     // (x(m) - x(m-1))^3 + (x(m+1) - x(m))^3
+  kPpmCoef
+};
+
 // interp Eq. (60)-(61) (rec.f90:1346-1418); the theta direction lacks the
 // factor 2 of r and phi (rec.f90:1414).
 template <typename T>
-__device__ __forceinline__ T ppm_dma(T um, T u0, T up, T dxm, T dx0, T dxp, bool kdir) {
-  const T t1a = dx0 / (dxm + dx0 + dxp);
-  const T t1b = (T(2.0) * dxm + dx0) / (dxp + dx0);
-  const T t1c = (dx0 + T(2.0) * dxp) / (dxm + dx0);
+__device__ __forceinline__ T ppm_dma(T um, T u0, T up, T ca, T cb, T cc, bool kdir) {
   const T sp1 = up - u0, sm1 = u0 - um;
   const T spm1 = sp1 * sm1;
-  const T da = t1a * (t1b * sp1 + t1c * sm1);
+  const T da = ca * (cb * sp1 + cc * sm1);
   if (spm1 <= T(0)) return T(0);
   const T t1 = (da < T(0)) ? T(-1) : T(1);
   const T t1d = dmin2(mabs(sm1), mabs(sp1));
@@ -306,98 +321,173 @@ __device__ __forceinline__ T ppm_dma(T um, T u0, T up, T dxm, T dx0, T dxp, bool
 
 // interp Eq. (51) (rec.f90:1422-1468): interface value at c+1/2.
 template <typename T>
-__device__ __forceinline__ T ppm_face(T u0, T u1, T dma0, T dma1, T dxm, T dx0, T dx1, T dx2) {
-  const T t2 = (dx0 / (dx0 + dx1)) * (u1 - u0);
-  const T t3a = T(1.0) / (dxm + dx0 + dx1 + dx2);
-  const T t3b = (T(2.0) * dx1 * dx0) / (dx0 + dx1);
-  const T t3c = ((dxm + dx0) / (T(2.0) * dx0 + dx1)) - ((dx2 + dx1) / (T(2.0) * dx1 + dx0));
-  const T t3 = t3a * t3b * t3c * (u1 - u0);
-  const T t4 = t3a * dx0 * ((dxm + dx0) / (T(2.0) * dx0 + dx1));
-  const T t5 = t3a * dx1 * ((dx1 + dx2) / (dx0 + T(2.0) * dx1));
+__device__ __forceinline__ T ppm_face(T u0, T u1, T dma0, T dma1, T t2c, T t3c, T t4, T t5) {
+  const T d = u1 - u0;
+  const T t2 = t2c * d;
+  const T t3 = t3c * d;
   return u0 + t2 + t3 - t4 * dma1 + t5 * dma0;
 }
 
-// Both face states of the cell at p (primitive v at p[v*N], storage type S),
-// stride st along direction D; dx[o+4], x[o+4] are the shifted spacing and
-// centre at offset o from the cell.  gam enters the contact test (rec.f90:1623).
-// ALL: also the sixth variable (the per-routine rec2 outputs every face state).
-// PACK: p holds the eight other variables one after another.
-template <int D, typename T, typename S, bool ALL = false, bool PACK = false>
-__device__ void ppm_cell(const S* __restrict__ p, size_t N, long long st, const T dx[9], const T x[9], T gam,
-                         T L[9], T R[9]) {
-  auto U = [&](int v, int o) { return T(p[(size_t)(PACK && v > 5 ? v - 1 : v) * N + o * st]); };
-  auto DX = [&](int o) { return dx[o + 4]; };
-  // detect (rec.f90:1479-1686): contact steepening factor eta on density
-  T eta;
+// a / b for a spacing b > 0 with its correctly rounded reciprocal rb
+__device__ __forceinline__ double ppm_over(double a, double b, double rb) {
+#ifdef RG_EXACT_ARITH
+  return a / b;
+#else
+  return div_by_rcp(a, b, rb);
+#endif
+}
+__device__ __forceinline__ float ppm_over(float a, float, float rb) { return a * rb; }
+
+// The contact steepening factor (detect, rec.f90:1479-1686) and the shock
+// flattening factor f2a (flaten, rec.f90:1689-1884) of the cell `o` cells above
+// the view's cell: U(v, o) the primitives, C(plane, o) the coefficients.
+// Quotients whose value cannot matter are not formed: the contact's pressure
+// test only where eta is not zero already (eta is never NaN), and a
+// flattening ratio only where its weight omg1 is one or the ratio could
+// overflow (0 * inf).
+template <int D, typename T, typename FU, typename FC>
+__device__ __forceinline__ void ppm_factors(const FU& U, const FC& C, int o, T gam, T& eta, T& f2a) {
+  const T pp = U(4, o + 1), pm = U(4, o - 1);
   {
     const T eta1 = T(5.0), eta2 = T(0.05), eps1 = T(0.1), ak0 = T(1.0);
-    auto dda = [&](int o) {
-      const T t0a = T(1.0) / (DX(o - 1) + DX(o) + DX(o + 1));
-      const T t0b = (U(0, o + 1) - U(0, o)) / (DX(o + 1) + DX(o));
-      const T t0c = (U(0, o) - U(0, o - 1)) / (DX(o) + DX(o - 1));
-      return t0a * (t0b - t0c);
+    auto dda = [&](int c) {
+      const T t0b = ppm_over(U(0, c + 1) - U(0, c), C(PC_S, c), C(PC_RS, c));
+      const T t0c = ppm_over(U(0, c) - U(0, c - 1), C(PC_S, c - 1), C(PC_RS, c - 1));
+      return C(PC_D, c) * (t0b - t0c);
     };
-    const T ddp = dda(1), ddm = dda(-1);
-    const T rp = U(0, 1), rm = U(0, -1);
+    const T ddp = dda(o + 1), ddm = dda(o - 1);
+    const T rp = U(0, o + 1), rm = U(0, o - 1);
     const T t1 = ddp * ddm;
     const T t2 = mabs(rp - rm) - eps1 * dmin2(mabs(rp), mabs(rm));
     T etatil;
     if (t1 >= T(0) && t2 <= T(0)) {
       etatil = T(0);
     } else {
-      const T t2a = -(ddp - ddm) / (x[5] - x[3]);
-      const T a = x[4] - x[3], b = x[5] - x[4];
-      const T t2b = (a * a * a + b * b * b) / (rp - rm);
+      const T t2a = -(ddp - ddm) / C(PC_X, o);
+      const T t2b = C(PC_X3, o) / (rp - rm);
       etatil = t2a * t2b;
     }
     eta = dmax2(T(0), dmin2(eta1 * (etatil - eta2), T(1)));
-    const T pp = U(4, 1), pm = U(4, -1);
-    const T t3 = mabs(rp - rm) / dmin2(rp, rm);
-    const T t4 = mabs(pp - pm) / dmin2(pp, pm);
-    if (gam * ak0 * t3 < t4) eta = T(0);
+    if (eta > T(0)) {
+      const T t3 = mabs(rp - rm) / dmin2(rp, rm);
+      const T t4 = mabs(pp - pm) / dmin2(pp, pm);
+      if (gam * ak0 * t3 < t4) eta = T(0);
+    }
   }
-  // flaten (rec.f90:1689-1884): shock flattening f2a from p and u^D
-  T f2a;
   {
     const T eps2 = T(1.0), omg2 = T(0.52), omg3 = T(10.0);
-    auto f1a = [&](int o) {
-      const T pp1 = U(4, o + 1), pm1 = U(4, o - 1);
+    const T tiny = sizeof(T) == 8 ? T(0x1p-1000) : T(0x1p-120f);
+    auto f1a = [&](int c) {
+      const T pp1 = U(4, c + 1), pm1 = U(4, c - 1);
       const T t3a = mabs(pp1 - pm1);
       const T t1 = eps2 * dmin2(pp1, pm1) - t3a;
-      const T t2 = U(D, o + 1) - U(D, o - 1);
+      const T t2 = U(D, c + 1) - U(D, c - 1);
       const T omg1 = (t1 < T(0) && t2 < T(0)) ? T(1) : T(0);
-      const T t3b = U(4, o + 2) - U(4, o - 2);
+      const T t3b = U(4, c + 2) - U(4, c - 2);
+      if (omg1 == T(0) && !(mabs(t3b) < t3a * tiny)) return T(0);
       T t4;
       if (t3b == T(0)) t4 = (t3a == T(0)) ? -omg2 : T(1.0) - omg2;
       else t4 = (t3a / t3b) - omg2;
       return dmin2(T(1), omg1 * dmax2(T(0), t4 * omg3));
     };
-    const T f1b = (U(4, 1) - U(4, -1) < T(0)) ? f1a(1) : f1a(-1);
-    f2a = dmax2(f1a(0), f1b);
+    const T f1b = (pp - pm < T(0)) ? f1a(o + 1) : f1a(o - 1);
+    f2a = dmax2(f1a(o), f1b);
   }
+}
+
+// flaten's blend and monoto (rec.f90:1887-2056) of one cell's states.
+template <typename T>
+__device__ __forceinline__ void ppm_monoto(T u0, T f2a, T& l, T& r) {
+  r = u0 * f2a + r * (T(1.0) - f2a);
+  l = u0 * f2a + l * (T(1.0) - f2a);
+  if ((r - u0) * (l - u0) >= T(0)) { r = u0; l = u0; }
+  const T t3 = T(6.0) * (r - l) * (u0 - T(0.5) * (r + l));
+  const T t4 = (r - l) * (r - l);
+  if (t3 > t4) l = T(3.0) * u0 - T(2.0) * r;
+  if (-t3 > t4) r = T(3.0) * u0 - T(2.0) * l;
+}
+
+// State of the cell at p (primitive v at p[v*N], storage type S), stride st
+// along direction D, at its upper (side 0) or lower (side 1) face; pc: the
+// coefficient planes at the cell's index, n apart.  gam enters the contact
+// test (rec.f90:1623).  ALL: also the sixth variable (the per-routine rec2
+// outputs every face state).
+template <int D, typename T, typename S, bool ALL>
+__device__ __forceinline__ void ppm_cell(const S* __restrict__ p, size_t N, long long st, const double* __restrict__ pc,
+                                         int n, T gam, int side, T q[9]) {
+  auto U = [&](int v, int o) { return T(p[(size_t)v * N + o * st]); };
+  auto C = [&](int a, int o) { return T(__ldg(pc + a * n + o)); };
+  T eta, f2a;
+  ppm_factors<D, T>(U, C, 0, gam, eta, f2a);
 #pragma unroll 1
   for (int v = 0; v < 9; ++v) {
-    if (v == 5 && !ALL) { L[v] = T(0); R[v] = T(0); continue; }  // var 6 faces are never read downstream
-    const T um2 = U(v, -2), um1 = U(v, -1), u0 = U(v, 0), up1 = U(v, 1), up2 = U(v, 2);
-    const T dm = ppm_dma(um2, um1, u0, DX(-2), DX(-1), DX(0), D == 3);
-    const T d0 = ppm_dma(um1, u0, up1, DX(-1), DX(0), DX(1), D == 3);
-    const T dp = ppm_dma(u0, up1, up2, DX(0), DX(1), DX(2), D == 3);
-    T l = ppm_face(um1, u0, dm, d0, DX(-2), DX(-1), DX(0), DX(1));
-    T r = ppm_face(u0, up1, d0, dp, DX(-1), DX(0), DX(1), DX(2));
-    if (v == 0) {
-      r = r * (T(1.0) - eta) + (up1 - T(0.5) * dp) * eta;
-      l = l * (T(1.0) - eta) + (um1 + T(0.5) * dm) * eta;
+    T o = T(0);
+    if (v != 5 || ALL) {  // var 6 faces are never read downstream
+      const T um2 = U(v, -2), um1 = U(v, -1), u0 = U(v, 0), up1 = U(v, 1), up2 = U(v, 2);
+      const T dm = ppm_dma(um2, um1, u0, C(PC_A, -1), C(PC_B, -1), C(PC_C, -1), D == 3);
+      const T d0 = ppm_dma(um1, u0, up1, C(PC_A, 0), C(PC_B, 0), C(PC_C, 0), D == 3);
+      const T dp = ppm_dma(u0, up1, up2, C(PC_A, 1), C(PC_B, 1), C(PC_C, 1), D == 3);
+      T l = ppm_face(um1, u0, dm, d0, C(PC_T2, -1), C(PC_T3, -1), C(PC_T4, -1), C(PC_T5, -1));
+      T r = ppm_face(u0, up1, d0, dp, C(PC_T2, 0), C(PC_T3, 0), C(PC_T4, 0), C(PC_T5, 0));
+      if (v == 0) {
+        r = r * (T(1.0) - eta) + (up1 - T(0.5) * dp) * eta;
+        l = l * (T(1.0) - eta) + (um1 + T(0.5) * dm) * eta;
+      }
+      ppm_monoto(u0, f2a, l, r);
+      o = side ? l : r;
     }
-    r = u0 * f2a + r * (T(1.0) - f2a);
-    l = u0 * f2a + l * (T(1.0) - f2a);
-    // monoto (rec.f90:1887-2056)
-    if ((r - u0) * (l - u0) >= T(0)) { r = u0; l = u0; }
-    const T t3 = T(6.0) * (r - l) * (u0 - T(0.5) * (r + l));
-    const T t4 = (r - l) * (r - l);
-    if (t3 > t4) l = T(3.0) * u0 - T(2.0) * r;
-    if (-t3 > t4) r = T(3.0) * u0 - T(2.0) * l;
-    L[v] = l;
-    R[v] = r;
+#pragma unroll
+    for (int w = 0; w < 9; ++w)
+      if (w == v) q[w] = o;
+  }
+}
+
+// Both states of one face by one thread: the upper state of the cell at p (L)
+// and the lower state of the next (R), which share two of their slopes and
+// the interface value between them.  PACK: p holds the eight variables other
+// than the sixth one after another.  put(v, L, R) receives each variable's
+// states; ROLL keeps the loop over the variables rolled (the 24 coefficients
+// then leave room in the registers; put must take a run-time v).
+template <int D, typename T, typename S, bool PACK, bool ROLL, typename Put>
+__device__ __forceinline__ void ppm_face_pair(const S* __restrict__ p, size_t N, long long st,
+                                              const double* __restrict__ pc, int n, T gam, const Put& put) {
+  auto U = [&](int v, int o) { return T(p[(size_t)(PACK && v > 5 ? v - 1 : v) * N + o * st]); };
+  auto C = [&](int a, int o) { return T(__ldg(pc + a * n + o)); };
+  T etaL, fL, etaR, fR;
+  ppm_factors<D, T>(U, C, 0, gam, etaL, fL);
+  ppm_factors<D, T>(U, C, 1, gam, etaR, fR);
+  T ca[4], cb[4], cc[4], t2[3], t3[3], t4[3], t5[3];
+#pragma unroll
+  for (int o = 0; o < 4; ++o) { ca[o] = C(PC_A, o - 1); cb[o] = C(PC_B, o - 1); cc[o] = C(PC_C, o - 1); }
+#pragma unroll
+  for (int o = 0; o < 3; ++o) { t2[o] = C(PC_T2, o - 1); t3[o] = C(PC_T3, o - 1); t4[o] = C(PC_T4, o - 1); t5[o] = C(PC_T5, o - 1); }
+  auto one = [&](int v) {
+    T u[6], d[4], f[3];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) u[o] = U(v, o - 2);
+#pragma unroll
+    for (int o = 0; o < 4; ++o) d[o] = ppm_dma(u[o], u[o + 1], u[o + 2], ca[o], cb[o], cc[o], D == 3);
+#pragma unroll
+    for (int o = 0; o < 3; ++o) f[o] = ppm_face(u[o + 1], u[o + 2], d[o], d[o + 1], t2[o], t3[o], t4[o], t5[o]);
+    T l0 = f[0], r0 = f[1], l1 = f[1], r1 = f[2];
+    if (v == 0) {
+      r0 = r0 * (T(1.0) - etaL) + (u[3] - T(0.5) * d[2]) * etaL;
+      l0 = l0 * (T(1.0) - etaL) + (u[1] + T(0.5) * d[0]) * etaL;
+      r1 = r1 * (T(1.0) - etaR) + (u[4] - T(0.5) * d[3]) * etaR;
+      l1 = l1 * (T(1.0) - etaR) + (u[2] + T(0.5) * d[1]) * etaR;
+    }
+    ppm_monoto(u[2], fL, l0, r0);
+    ppm_monoto(u[3], fR, l1, r1);
+    put(v, r0, l1);
+  };
+  if constexpr (ROLL) {
+#pragma unroll 1
+    for (int v = 0; v < 9; ++v)
+      if (v != 5) one(v);  // var 6 faces are never read downstream
+  } else {
+#pragma unroll
+    for (int v = 0; v < 9; ++v)
+      if (v != 5) one(v);
   }
 }
 

@@ -20,6 +20,8 @@ constexpr int NV = 9;
 // kMetBase (gcov, gcon blocks, sqrt(-g)); k_met_derive fills the rest.
 constexpr int kMetBase = 18;
 constexpr int kMetComps = 26;
+// Planes of PPM's coefficient tables (PpmCoef in rg_recon.cuh).
+constexpr int kPpmPlanes = 12;
 
 // Planes of the torus initial-data table (TorusTables): per radial index,
 // then per theta index.
@@ -80,8 +82,6 @@ struct DevRun {
   const double* dx1b;    // dx1b(i) at index i-1 (grid.f90:134-141)
   const double* dx2b;
   const double* dx3b;
-  const double* x2;      // phi centres (PPM contact detection)
-  const double* x3;      // theta centres
   const double* fl_de;   // density floor dmin * x1(i)**(-1.5) (correction.f90:897), index i-1
   const double* fl_pr;   // pressure floor (gam-1) * pmin * x1(i)**(-2.5) (correction.f90:898), index i-1
   double* Un;            // conserved variables of the step's initial primitives (9*N), written in stage 1
@@ -93,9 +93,9 @@ struct DevRun {
   float* P32;            // FP32 copy of the current primitives (written by the floor pass)
   float* F32[3];         // FP32 face fluxes per direction, 9*N each
   float* CT32;           // FP32 flux-CT values, 6*N
-  const double* dx1s;    // rec2's shifted dx1b: dummy dx1b(i) = actual dx1b(i-1), index i-1
-  const double* dx2s;
-  const double* dx3s;
+  // PPM's coefficients of the spacings per direction (PpmCoef in rg_recon.cuh,
+  // kPpmCoef planes of n_d values at index m-1; only for irec 5)
+  const double* ppm[3];
   // Limiter coefficients per direction d (MC, minmod, LimO3, MVL, Koren,
   // CENO): ten planes of n_d values at index m-1 of the cell's coordinate
   // spacings, as limiter_state and ceno_state in rg_recon.cuh read them.
