@@ -92,6 +92,34 @@ __device__ __forceinline__ T mp5_value(T a2, T a1, T u0, T b1, T b2) {
 #endif
 }
 
+// The convex combination of the three candidates with the weights n_m / d_m
+// as the reference forms it: six quotients.
+#ifdef RG_EXACT_ARITH
+#define RG_WENO_QUOT __forceinline__
+#else
+#define RG_WENO_QUOT __noinline__
+#endif
+template <typename T>
+__device__ RG_WENO_QUOT T weno_quot(T n0, T d0, T n1, T d1, T n2, T d2, T q0, T q1, T q2) {
+  const T w0 = n0 / d0, w1 = n1 / d1, w2 = n2 / d2;
+  const T wt = w0 + w1 + w2;
+  const T o0 = w0 / wt, o1 = w1 / wt, o2 = w2 / wt;
+  return o0 * q0 + o1 * q1 + o2 * q2;
+}
+// The same with weights already multiplied by their common denominator, which
+// leaves one reciprocal.  Where the products leave the range in which they
+// and the reciprocal are exact to rounding (fields beyond about 1e37 in FP64 or
+// 1e4 in FP32, non-finite values), `quot` forms the quotients instead.
+template <typename T, typename F>
+__device__ __forceinline__ T weno_mean(T w0, T w1, T w2, T q0, T q1, T q2, const F& quot) {
+  const T wt = w0 + w1 + w2;
+  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p120f), small = sizeof(T) == 8 ? T(0x1p-500) : T(0x1p-100f);
+  if (!(wt < big && wt > small)) return quot();
+  const T o = w0 * q0 + w1 * q1 + w2 * q2;
+  if constexpr (sizeof(T) == 8) return o * rcp_newton(wt);
+  else return mdiv(o, wt);
+}
+
 // rec.f90:2373-2643 (WENO5-JS); the left state at +1/2 takes
 // (u-2, u-1, u0, u+1, u+2), the right state at -1/2 the mirrored stencil.
 // (13./12.) is a single-precision literal in the reference.
@@ -110,13 +138,20 @@ __device__ __forceinline__ T weno5_js(T a2, T a1, T u0, T b1, T b2, T b1s) {
   const T be0 = c1312 * (s0 * s0) + c14 * (t0 * t0) + epsi;
   const T be1 = c1312 * (s1 * s1) + c14 * (t1 * t1) + epsi;
   const T be2 = c1312 * (s2 * s2) + c14 * (t2 * t2) + epsi;
-  const T w0 = cd0 / (be0 * be0), w1 = cd1 / (be1 * be1), w2 = cd2 / (be2 * be2);
-  const T wt = w0 + w1 + w2;
-  const T o0 = w0 / wt, o1 = w1 / wt, o2 = w2 / wt;
   const T q0 = c00 * a2 + c01 * a1 + c02 * u0;
   const T q1 = c10 * a1 + c11 * u0 + c12 * b1;
   const T q2 = c20 * u0 + c21 * b1 + c22 * b2;
-  return o0 * q0 + o1 * q1 + o2 * q2;
+#ifndef RG_EXACT_ARITH
+  {
+    // the weights cd_m / beta_m^2 times (beta_0 beta_1 beta_2)^2
+    const T p0 = be1 * be2, p1 = be0 * be2, p2 = be0 * be1;
+    return weno_mean(cd0 * (p0 * p0), cd1 * (p1 * p1), cd2 * (p2 * p2), q0, q1, q2, [&] {
+      return weno_quot(cd0, be0 * be0, cd1, be1 * be1, cd2, be2 * be2, q0, q1, q2);
+    });
+  }
+#else
+  return weno_quot(cd0, be0 * be0, cd1, be1 * be1, cd2, be2 * be2, q0, q1, q2);
+#endif
 }
 template <typename T>
 __device__ __forceinline__ T weno5_state(T a2, T a1, T u0, T b1, T b2) {
@@ -140,15 +175,25 @@ __device__ __forceinline__ T weno5z_state(T a2, T a1, T u0, T b1, T b2) {
   const T be1 = c1312 * (s1 * s1) + c14 * (t1 * t1);
   const T be2 = c1312 * (s2 * s2) + c14 * (t2 * t2);
   const T tau = mabs(be0 - be2);
-  const T w0 = cd0 * (T(1.0) + tau / (be0 + epsi));
-  const T w1 = cd1 * (T(1.0) + tau / (be1 + epsi));
-  const T w2 = cd2 * (T(1.0) + tau / (be2 + epsi));
-  const T wt = w0 + w1 + w2;
-  const T o0 = w0 / wt, o1 = w1 / wt, o2 = w2 / wt;
   const T q0 = c00 * a2 + c01 * a1 + c02 * u0;
   const T q1 = c10 * a1 + c11 * u0 + c12 * b1;
   const T q2 = c20 * u0 + c21 * b1 + c22 * b2;
-  return o0 * q0 + o1 * q1 + o2 * q2;
+  auto quot = [&] {
+    const T w0 = cd0 * (T(1.0) + tau / (be0 + epsi));
+    const T w1 = cd1 * (T(1.0) + tau / (be1 + epsi));
+    const T w2 = cd2 * (T(1.0) + tau / (be2 + epsi));
+    const T wt = w0 + w1 + w2;
+    const T o0 = w0 / wt, o1 = w1 / wt, o2 = w2 / wt;
+    return o0 * q0 + o1 * q1 + o2 * q2;
+  };
+#ifndef RG_EXACT_ARITH
+  // the weights times the product of the beta_m + eps
+  const T e0 = be0 + epsi, e1 = be1 + epsi, e2 = be2 + epsi;
+  return weno_mean(cd0 * (e0 + tau) * (e1 * e2), cd1 * (e1 + tau) * (e0 * e2), cd2 * (e2 + tau) * (e0 * e1), q0, q1,
+                   q2, quot);
+#else
+  return quot();
+#endif
 }
 
 // rec.f90:3439-3793 (mapped WENO5, Henrick et al. 2005): the JS weights
@@ -167,21 +212,47 @@ __device__ __forceinline__ T weno5m_state(T a2, T a1, T u0, T b1, T b2) {
   const T s2 = u0 - T(2.) * b1 + b2, t2 = T(3.) * u0 - T(4.) * b1 + b2;
   const T be[3] = {c1312 * (s0 * s0) + c14 * (t0 * t0), c1312 * (s1 * s1) + c14 * (t1 * t1),
                    c1312 * (s2 * s2) + c14 * (t2 * t2)};
-  T wa[3], g[3];
-#pragma unroll
-  for (int m = 0; m < 3; ++m) wa[m] = cd[m] / ((be[m] + epsi) * (be[m] + epsi));
-  const T wat = wa[0] + wa[1] + wa[2];
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const T w = wa[m] / wat;
-    g[m] = w * (cd[m] + cd[m] * cd[m] - T(3.) * cd[m] * w + w * w) / (cd[m] * cd[m] + w * (T(1.) - T(2.) * cd[m]));
-  }
-  const T gt = g[0] + g[1] + g[2];
-  const T o0 = g[0] / gt, o1 = g[1] / gt, o2 = g[2] / gt;
   const T q0 = c00 * a2 + c01 * a1 + c02 * u0;
   const T q1 = c10 * a1 + c11 * u0 + c12 * b1;
   const T q2 = c20 * u0 + c21 * b1 + c22 * b2;
-  return o0 * q0 + o1 * q1 + o2 * q2;
+  auto quot = [&] {
+    T wa[3], g[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) wa[m] = cd[m] / ((be[m] + epsi) * (be[m] + epsi));
+    const T wat = wa[0] + wa[1] + wa[2];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const T w = wa[m] / wat;
+      g[m] = w * (cd[m] + cd[m] * cd[m] - T(3.) * cd[m] * w + w * w) / (cd[m] * cd[m] + w * (T(1.) - T(2.) * cd[m]));
+    }
+    const T gt = g[0] + g[1] + g[2];
+    const T o0 = g[0] / gt, o1 = g[1] / gt, o2 = g[2] / gt;
+    return o0 * q0 + o1 * q1 + o2 * q2;
+  };
+#ifndef RG_EXACT_ARITH
+  if constexpr (sizeof(T) == 8) {
+    // the weights times (beta_0 + eps)^2 (beta_1 + eps)^2 (beta_2 + eps)^2, the
+    // beta_m + eps (at least 1e-40) scaled by 2^60 to keep the products from
+    // underflowing; the mapped weights over their common denominator
+    const T sc = T(0x1p60);
+    const T e0 = sc * (be[0] + epsi), e1 = sc * (be[1] + epsi), e2 = sc * (be[2] + epsi);
+    const T p0 = e1 * e2, p1 = e0 * e2, p2 = e0 * e1;
+    const T w[3] = {cd[0] * (p0 * p0), cd[1] * (p1 * p1), cd[2] * (p2 * p2)};
+    const T wt = w[0] + w[1] + w[2];
+    if (!(wt < T(0x1p500) && wt > T(0x1p-500))) return quot();
+    const T iw = rcp_newton(wt);
+    T num[3], den[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const T o = w[m] * iw;
+      num[m] = o * (cd[m] + cd[m] * cd[m] - T(3.) * cd[m] * o + o * o);
+      den[m] = cd[m] * cd[m] + o * (T(1.) - T(2.) * cd[m]);
+    }
+    return weno_mean(num[0] * (den[1] * den[2]), num[1] * (den[0] * den[2]), num[2] * (den[0] * den[1]), q0, q1, q2,
+                     quot);
+  }
+#endif
+  return quot();
 }
 
 // The second-order limiters of rec.f90 on nonuniform coordinates: mclim
