@@ -14,13 +14,20 @@
 // device (Scal::cur), which makes one step's launch sequence valid for every
 // step: the host captures it once in a CUDA graph and replays it.
 
+// Resident blocks per SM the batched FP64 face kernel is compiled for.
+#ifndef RG_BATCH_FLUX_MINB64
+#define RG_BATCH_FLUX_MINB64 4
+#endif
+
 namespace {
 
 // nsub: the tile covers blocks bx .. bx+nsub-1 of the run's grid (the tile
-// shape along i is nsub blocks of the cell kernels' width).
+// shape along i is nsub blocks of the cell kernels' width); dir: the direction
+// of a face tile.
 struct Tile {
   int run, bx, by, bz;
-  int ilo, ihi, aux, nsub;
+  int ilo, ihi, aux;
+  short nsub, dir;
 };
 
 // P^n, the stage input and the stage output of a run (stage 0: CFL, P^n only).
@@ -53,17 +60,26 @@ __global__ void __launch_bounds__(NT, MINB) kb(const DevRun* __restrict__ runs, 
   }
 }
 
-template <int D, int IREC, typename T, typename S>
+// The faces of all three directions in one launch, the direction from the tile:
+// they are independent, and on the small grids of a batch each alone is a few
+// rounds of blocks that ends in an empty one.
+template <int IREC, typename T, typename S>
 struct FluxB {
   int stage;
-  __device__ void operator()(const DevRun& r, const Tile& t) const {
-    double *Pn, *Pc, *Pw;
-    stage_ptrs(r, stage, Pn, Pc, Pw);
+  template <int D>
+  __device__ __forceinline__ void dir(const DevRun& r, const Tile& t, const double* Pc) const {
     if constexpr (sizeof(S) == 8)
       flux_body<D, IREC, T, S>(r, Pc, r.F[D - 1], r.mixed ? r.F32[D - 1] : nullptr, t.aux, t.ilo, t.ihi,
                                make_uint3(t.bx, t.by, t.bz));
     else
       flux_body<D, IREC, T, S>(r, r.P32, r.F32[D - 1], nullptr, 0, t.ilo, t.ihi, make_uint3(t.bx, t.by, t.bz));
+  }
+  __device__ void operator()(const DevRun& r, const Tile& t) const {
+    double *Pn, *Pc, *Pw;
+    stage_ptrs(r, stage, Pn, Pc, Pw);
+    if (t.dir == 1) dir<1>(r, t, Pc);
+    else if (t.dir == 2) dir<2>(r, t, Pc);
+    else dir<3>(r, t, Pc);
   }
 };
 
@@ -112,8 +128,9 @@ struct BcB {
   __device__ void operator()(const DevRun& r, const Tile& t) const {
     double *Pn, *Pc, *Pw;
     stage_ptrs(r, stage, Pn, Pc, Pw);
-    if (PERIODIC) bc_periodic_body<D>(r, Pw, make_uint3(t.bx, t.by, t.bz));
-    else bc_phys_body<D>(r, Pw, Pn, make_uint3(t.bx, t.by, t.bz));
+    // one variable per z index of the grid, as the single-run passes take it
+    if (PERIODIC) bc_periodic_body<D>(r, Pw, make_uint3(t.bx, t.by, 0), t.bz, t.bz + 1);
+    else bc_phys_body<D>(r, Pw, Pn, make_uint3(t.bx, t.by, 0), t.bz, t.bz + 1);
   }
 };
 
@@ -175,11 +192,12 @@ struct BatchPlan {
 
 namespace {
 
-inline void add_tiles(std::vector<Tile>& T, int run, dim3 g, int ilo, int ihi, int aux, int group = 1) {
+inline void add_tiles(std::vector<Tile>& T, int run, dim3 g, int ilo, int ihi, int aux, int group = 1, int dir = 0) {
   for (unsigned z = 0; z < g.z; ++z)
     for (unsigned y = 0; y < g.y; ++y)
       for (unsigned x = 0; x < g.x; x += (unsigned)group)
-        T.push_back(Tile{run, (int)x, (int)y, (int)z, ilo, ihi, aux, (int)std::min<unsigned>(group, g.x - x)});
+        T.push_back(Tile{run, (int)x, (int)y, (int)z, ilo, ihi, aux, (short)std::min<unsigned>(group, g.x - x),
+                         (short)dir});
 }
 
 // Block shape of a cell kernel in a batch of slab runs: `width` threads along i.
@@ -235,31 +253,30 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, BatchPlan
   plan_append(*B, T, L, runs, one);
   for (int stage = 1; stage <= 3; ++stage) {
     L.stage = stage;
-    for (int dir = 1; dir <= 3; ++dir) {
-      L.kind = BK_FLUX;
-      L.dir = dir;
-      L.block = wblock(r0, dim3(64, 2, 1), width);
-      for (int part = 0; part < 2; ++part) {
-        L.fp32 = part;
-        plan_append(*B, T, L, runs, [&](int a, const DevRun& r, std::vector<Tile>& t) {
-          const int lo = r.nm0, hi = r.imax - r.nm0, m = r.jmax - 2 * r.nm0 + 1, l = r.kmax - 2 * r.nm0 + 1;
-          int ilo = lo, ihi = hi, aux = 0;
-          if (!r.mixed) {
-            if (part == 1) return;
+    L.kind = BK_FLUX;
+    L.dir = 0;
+    L.block = wblock(r0, dim3(64, 2, 1), width);
+    for (int part = 0; part < 2; ++part) {
+      L.fp32 = part;
+      plan_append(*B, T, L, runs, [&](int a, const DevRun& r, std::vector<Tile>& t) {
+        const int lo = r.nm0, hi = r.imax - r.nm0, m = r.jmax - 2 * r.nm0 + 1, l = r.kmax - 2 * r.nm0 + 1;
+        int ilo = lo, ihi = hi, aux = 0;
+        if (!r.mixed) {
+          if (part == 1) return;
+        } else {
+          const int split = fp64_split(r, lo, hi);
+          if (part == 0) {
+            if (split < lo) return;
+            ihi = split < hi ? split + 1 : hi;
+            aux = split;
           } else {
-            const int split = fp64_split(r, lo, hi);
-            if (part == 0) {
-              if (split < lo) return;
-              ihi = split < hi ? split + 1 : hi;
-              aux = split;
-            } else {
-              if (split >= hi) return;
-              ilo = split + 1;
-            }
+            if (split >= hi) return;
+            ilo = split + 1;
           }
-          add_tiles(t, a, sgrid(r, 2 * (ihi - ilo + 1), m, l, L.block), ilo, ihi, aux, group);
-        });
-      }
+        }
+        for (int dir = 1; dir <= 3; ++dir)
+          add_tiles(t, a, sgrid(r, 2 * (ihi - ilo + 1), m, l, L.block), ilo, ihi, aux, group, dir);
+      });
     }
     L.kind = BK_CT;
     L.dir = 0;
@@ -313,7 +330,7 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, BatchPlan
         const bool slab = (dir == 2 && jf) || (dir == 3 && kf);
         if (slab) continue;
         const bool fix1 = (dir == 1) ? jf : false, fix2 = (dir == 3) ? jf : kf;
-        bc_shape(8, 8, fix1, fix2, g, b);
+        bc_shape9(8, 8, fix1, fix2, g, b);
         L.block = b;
         plan_append(*B, T, L, runs, [&](int a, const DevRun& r, std::vector<Tile>& t) {
           if (!any_code(r, 2 * (dir - 1), per != 0)) return;
@@ -324,7 +341,7 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, BatchPlan
           else { n1 = r.imax; n2 = r.jmax; }
           if (per) { n1 -= 2 * nm1; n2 -= 2 * nm1; }
           dim3 gg, bb;
-          bc_shape(n1, n2, fix1, fix2, gg, bb);
+          bc_shape9(n1, n2, fix1, fix2, gg, bb);
           add_tiles(t, a, gg, 0, 0, 0);
         });
       }
@@ -388,36 +405,29 @@ cudaError_t kb_go(const BatchPlan* B, const BLaunch& L, Body body, cudaStream_t 
 // so a run's cells go through the same compiled code alone and in any mix;
 // MINB keeps each kernel's register budget of the single-run launch (FP64
 // faces 96, FP32 faces 64, update 168 registers).
-template <int D, int IREC, typename T, typename S>
+template <int IREC, typename T, typename S>
 cudaError_t go_flux(const BatchPlan* B, const BLaunch& L, cudaStream_t s) {
-  const FluxB<D, IREC, T, S> b{L.stage};
-  return kb_go<FluxB<D, IREC, T, S>, 128, sizeof(T) == 8 ? RG_FLUX_MINB64 : 8>(B, L, b, s);
-}
-
-template <int D, typename T, typename S>
-cudaError_t go_flux_irec(const BatchPlan* B, const BLaunch& L, cudaStream_t s) {
-  switch (B->irec) {
-    case 1: return go_flux<D, 1, T, S>(B, L, s);
-    case 2: return go_flux<D, 2, T, S>(B, L, s);
-    case 3: return go_flux<D, 3, T, S>(B, L, s);
-    case 4: return go_flux<D, 4, T, S>(B, L, s);
-    case 8: return go_flux<D, 8, T, S>(B, L, s);
-    case 10: return go_flux<D, 10, T, S>(B, L, s);
-    case 11: return go_flux<D, 11, T, S>(B, L, s);
-    case 12: return go_flux<D, 12, T, S>(B, L, s);
-    case 13: return go_flux<D, 13, T, S>(B, L, s);
-    case 5: return go_flux<D, 5, T, S>(B, L, s);
-    case 6: return go_flux<D, 6, T, S>(B, L, s);
-    case 7: return go_flux<D, 7, T, S>(B, L, s);
-    default: return go_flux<D, 9, T, S>(B, L, s);
-  }
+  const FluxB<IREC, T, S> b{L.stage};
+  return kb_go<FluxB<IREC, T, S>, 128, sizeof(T) == 8 ? RG_BATCH_FLUX_MINB64 : 8>(B, L, b, s);
 }
 
 template <typename T, typename S>
-cudaError_t go_flux_dir(const BatchPlan* B, const BLaunch& L, cudaStream_t s) {
-  if (L.dir == 1) return go_flux_irec<1, T, S>(B, L, s);
-  if (L.dir == 2) return go_flux_irec<2, T, S>(B, L, s);
-  return go_flux_irec<3, T, S>(B, L, s);
+cudaError_t go_flux_irec(const BatchPlan* B, const BLaunch& L, cudaStream_t s) {
+  switch (B->irec) {
+    case 1: return go_flux<1, T, S>(B, L, s);
+    case 2: return go_flux<2, T, S>(B, L, s);
+    case 3: return go_flux<3, T, S>(B, L, s);
+    case 4: return go_flux<4, T, S>(B, L, s);
+    case 5: return go_flux<5, T, S>(B, L, s);
+    case 6: return go_flux<6, T, S>(B, L, s);
+    case 7: return go_flux<7, T, S>(B, L, s);
+    case 8: return go_flux<8, T, S>(B, L, s);
+    case 10: return go_flux<10, T, S>(B, L, s);
+    case 11: return go_flux<11, T, S>(B, L, s);
+    case 12: return go_flux<12, T, S>(B, L, s);
+    case 13: return go_flux<13, T, S>(B, L, s);
+    default: return go_flux<9, T, S>(B, L, s);
+  }
 }
 
 template <int STAGE, bool MIX>
@@ -447,7 +457,7 @@ cudaError_t batch_issue(const BatchPlan* B, int idx, cudaStream_t s) {
     case BK_END: return kb_go<ScalarB<2>, 32, 1>(B, L, ScalarB<2>{}, s);
     case BK_CFL: return go_cell(B, L, CflB{}, s);
     case BK_FLUX:
-      return L.fp32 ? go_flux_dir<float, float>(B, L, s) : go_flux_dir<double, double>(B, L, s);
+      return L.fp32 ? go_flux_irec<float, float>(B, L, s) : go_flux_irec<double, double>(B, L, s);
     case BK_CT:
       if (B->ict == 0)
         return L.fp32 ? go_cell(B, L, CtB<0, float, float>{}, s) : go_cell(B, L, CtB<0, double, double>{}, s);

@@ -708,7 +708,7 @@ int kind_of(const BatchPlan* B, int idx) {
   int dir = 0;
   switch (batch_launch_kind(B, idx, &dir)) {
     case 1: return K_CFL;
-    case 3: return K_FLUX1 + dir - 1;
+    case 3: return K_FLUX1;  // one launch for the faces of all directions
     case 4: return K_CT;
     case 5: case 6: return K_UPDATE;
     case 7: case 8: return K_BC;
