@@ -53,7 +53,6 @@ struct Run {
   // calls never touch the run's own time state, buffer rotation or statistics
   Scal* fscal = nullptr;
   unsigned long long* fcnt = nullptr;
-  int* bad = nullptr;      // device flag: uploaded data not uniform along a slab direction
   size_t nfull = 0;        // imax*jmax*kmax
   int cur = 0;             // index of P^n in b.P
   std::vector<void*> allocs;
@@ -114,6 +113,7 @@ struct rg_ctx {
   double ms[K_NKINDS] = {};
   bool own_stream = true;              // false after rg_ctx_set_stream
   cudaEvent_t marks[RG_MAX_MARKS] = {};  // rg_ctx_mark / rg_ctx_wait_mark
+  int* flag = nullptr;                 // one word of pinned host memory that kernels write (uploaded data not uniform)
   bool tma = true;                     // staged face kernel where a run allows it (RAISHIN_FLUX_TMA=0: off)
   bool utma = true;                    // staged update kernel where a run allows it (RAISHIN_UPDATE_TMA=0: off)
 };
@@ -454,7 +454,7 @@ int reset_fscal(rg_ctx* ctx, Run* R, double dtcfl0 = 0.0) {
   Scal sc{};
   sc.active = 1;
   std::memcpy(&sc.dtcfl_bits, &dtcfl0, sizeof(double));
-  RG_CUDA(cudaMemcpyAsync(R->fscal, &sc, sizeof(Scal), cudaMemcpyHostToDevice, ctx->stream));
+  RG_CUDA(launch_set_scal(R->fscal, sc, ctx->stream));
   return RG_OK;
 }
 
@@ -509,8 +509,19 @@ int set_time(rg_ctx* ctx, Run* R, double t0) {
   s.timeh = t0;
   s.active = 1;
   s.carry_count = 0;
-  RG_CUDA(cudaMemcpyAsync(R->d.scal, &s, sizeof(Scal), cudaMemcpyHostToDevice, ctx->stream));
+  RG_CUDA(launch_set_scal(R->d.scal, s, ctx->stream));
   return RG_OK;
+}
+
+// Whether a kernel of this context may read or write p in place: memory of its
+// device, aligned for doubles (anything else is staged by a copy).
+bool device_array(const rg_ctx* ctx, const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == ctx->device && reinterpret_cast<uintptr_t>(p) % 8 == 0;
 }
 
 int ensure_aos(Run* R) {
@@ -526,18 +537,21 @@ int ensure_aos(Run* R) {
 // stored layout, or the full layout of the per-routine entry points).  With
 // check, data that are not uniform along a slab direction are refused.
 int to_soa(rg_ctx* ctx, Run* R, const double* host_aos, double* dev_soa, const DevRun& v, bool check) {
-  int rc = ensure_aos(R);
-  if (rc) return rc;
-  // cudaMemcpyDefault: the caller's array may be host memory or device memory (unified addressing)
-  RG_CUDA(cudaMemcpyAsync(R->aos, host_aos, 9 * R->nfull * sizeof(double), cudaMemcpyDefault, ctx->stream));
-  const bool slab = v.jfix || v.kfix;
-  if (check && slab) RG_CUDA(cudaMemsetAsync(R->bad, 0, sizeof(int), ctx->stream));
-  RG_CUDA(launch_aos_to_soa(v, R->aos, dev_soa, (check && slab) ? R->bad : nullptr, ctx->stream));
-  if (check && slab) {
-    int bad = 0;
-    RG_CUDA(cudaMemcpyAsync(&bad, R->bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  // an array on this device is read where it is; any other is copied to the
+  // run's staging buffer first (cudaMemcpyDefault: host memory or another device's)
+  const double* src = host_aos;
+  if (!device_array(ctx, host_aos)) {
+    const int rc = ensure_aos(R);
+    if (rc) return rc;
+    RG_CUDA(cudaMemcpyAsync(R->aos, host_aos, 9 * R->nfull * sizeof(double), cudaMemcpyDefault, ctx->stream));
+    src = R->aos;
+  }
+  const bool verify = check && (v.jfix || v.kfix);
+  if (verify) *ctx->flag = 0;
+  RG_CUDA(launch_aos_to_soa(v, src, dev_soa, verify ? ctx->flag : nullptr, ctx->stream));
+  if (verify) {
     RG_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (bad)
+    if (*static_cast<volatile int*>(ctx->flag))
       return fail(RG_EINVAL_CONFIG,
                   "primitives differ along a slab direction (the run stores one plane of it); admit the run "
                   "with flags bit 0 (RG_FLAG_FULL) to compute every cell");
@@ -546,10 +560,14 @@ int to_soa(rg_ctx* ctx, Run* R, const double* host_aos, double* dev_soa, const D
 }
 
 int from_soa(rg_ctx* ctx, Run* R, const double* dev_soa, double* host_aos, const DevRun& v) {
-  int rc = ensure_aos(R);
-  if (rc) return rc;
-  RG_CUDA(launch_soa_to_aos(v, dev_soa, R->aos, ctx->stream));
-  RG_CUDA(cudaMemcpyAsync(host_aos, R->aos, 9 * R->nfull * sizeof(double), cudaMemcpyDefault, ctx->stream));
+  if (device_array(ctx, host_aos)) {
+    RG_CUDA(launch_soa_to_aos(v, dev_soa, host_aos, ctx->stream));
+  } else {
+    const int rc = ensure_aos(R);
+    if (rc) return rc;
+    RG_CUDA(launch_soa_to_aos(v, dev_soa, R->aos, ctx->stream));
+    RG_CUDA(cudaMemcpyAsync(host_aos, R->aos, 9 * R->nfull * sizeof(double), cudaMemcpyDefault, ctx->stream));
+  }
   RG_CUDA(cudaStreamSynchronize(ctx->stream));
   return RG_OK;
 }
@@ -913,8 +931,10 @@ int rg_ctx_create(int device, rg_ctx** out) {
   c->device = device;
   if (const char* t = std::getenv("RAISHIN_FLUX_TMA")) c->tma = std::strcmp(t, "0") != 0;
   if (const char* t = std::getenv("RAISHIN_UPDATE_TMA")) c->utma = std::strcmp(t, "0") != 0;
-  cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+  cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&c->flag), sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
+    cudaFreeHost(c->flag);
     delete c;
     return fail(RG_ECUDA, cudaGetErrorString(e));
   }
@@ -933,6 +953,7 @@ int rg_ctx_destroy(rg_ctx* ctx) {
   for (cudaEvent_t e : ctx->marks)
     if (e) cudaEventDestroy(e);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
+  cudaFreeHost(ctx->flag);
   delete ctx;
   return RG_OK;
 }
@@ -1109,8 +1130,6 @@ int rg_run_admit_prep(rg_ctx* ctx, rg_prep* prep, int* run_id) {
   }
   if ((rc = dalloc(R, &ptr, 9 * N * sizeof(double)))) return bail(rc);
   d.Un = static_cast<double*>(ptr);
-  if ((rc = dalloc(R, &ptr, sizeof(int)))) return bail(rc);
-  R->bad = static_cast<int*>(ptr);
   if (!d.jfix && !d.kfix) {  // the full layout is the stored one: share the step's flux buffers
     R->fb.F[0] = R->b.F[0]; R->fb.F[1] = R->b.F[1]; R->fb.F[2] = R->b.F[2]; R->fb.CT = R->b.CT;
   }

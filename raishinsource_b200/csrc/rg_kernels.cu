@@ -2612,38 +2612,42 @@ __global__ void __launch_bounds__(128) k_rkt(DevRun r, const double* __restrict_
 // stored cells' values and flags (bad != 0) any full-array cell whose value
 // differs from the stored cell it maps to: a slab direction holds one plane,
 // so its data must be uniform along it.  Download writes every full cell.
-__global__ void k_aos_to_soa(DevRun r, const double* __restrict__ a, double* __restrict__ s, int* bad) {
-  const size_t f = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t nfull = (size_t)r.imax * r.jmax * r.kmax;
+// (bad may be mapped host memory: it is only stored to.)
+__global__ void k_aos_to_soa(DevRun r, const double* __restrict__ a, double* __restrict__ s, volatile int* bad) {
+  const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;  // at most 1.9e9 cells (check_params)
+  const unsigned nfull = (unsigned)r.imax * (unsigned)r.jmax * (unsigned)r.kmax;
   if (f >= nfull) return;
-  const int i = (int)(f % r.imax) + 1;
-  const int j = (int)((f / r.imax) % r.jmax) + 1;
-  const int k = (int)(f / ((size_t)r.imax * r.jmax)) + 1;
+  const unsigned row = f / (unsigned)r.imax;
+  const int i = (int)(f - row * (unsigned)r.imax) + 1;
+  const int k = (int)(row / (unsigned)r.jmax) + 1;
+  const int j = (int)(row - (unsigned)(k - 1) * (unsigned)r.jmax) + 1;
   const bool owner = (!r.jfix || j == r.jfix) && (!r.kfix || k == r.kfix);
   const size_t c = r.cell(i, j, k);
   if (owner) {
 #pragma unroll
-    for (int v = 0; v < 9; ++v) s[(size_t)v * r.N + c] = a[9 * f + v];
+    for (int v = 0; v < 9; ++v) s[(size_t)v * r.N + c] = a[9 * (size_t)f + v];
   } else if (bad) {
     const size_t o = r.cell_full(i, r.jfix ? r.jfix : j, r.kfix ? r.kfix : k);
     bool same = true;
 #pragma unroll
     for (int v = 0; v < 9; ++v)
-      same = same && (__double_as_longlong(a[9 * f + v]) == __double_as_longlong(a[9 * o + v]));
-    if (!same) atomicOr(bad, 1);
+      same = same && (__double_as_longlong(a[9 * (size_t)f + v]) == __double_as_longlong(a[9 * o + v]));
+    if (!same) *bad = 1;
   }
 }
 __global__ void k_soa_to_aos(DevRun r, const double* __restrict__ s, double* __restrict__ a) {
-  const size_t f = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t nfull = (size_t)r.imax * r.jmax * r.kmax;
+  const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned nfull = (unsigned)r.imax * (unsigned)r.jmax * (unsigned)r.kmax;
   if (f >= nfull) return;
-  const int i = (int)(f % r.imax) + 1;
-  const int j = (int)((f / r.imax) % r.jmax) + 1;
-  const int k = (int)(f / ((size_t)r.imax * r.jmax)) + 1;
+  const unsigned row = f / (unsigned)r.imax;
+  const int i = (int)(f - row * (unsigned)r.imax) + 1;
+  const int k = (int)(row / (unsigned)r.jmax) + 1;
+  const int j = (int)(row - (unsigned)(k - 1) * (unsigned)r.jmax) + 1;
   const size_t c = r.cell(i, j, k);
 #pragma unroll
-  for (int v = 0; v < 9; ++v) a[9 * f + v] = s[(size_t)v * r.N + c];
+  for (int v = 0; v < 9; ++v) a[9 * (size_t)f + v] = s[(size_t)v * r.N + c];
 }
+__global__ void k_set_scal(Scal* dst, Scal v) { *dst = v; }
 __global__ void k_fill(double* p, double v, size_t n) {
   const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c < n) p[c] = v;
@@ -3260,6 +3264,10 @@ cudaError_t launch_rkt(const DevRun& r, int stage, const double* W1, const doubl
   return cudaGetLastError();
 }
 
+cudaError_t launch_set_scal(Scal* dst, const Scal& v, cudaStream_t s) {
+  k_set_scal<<<1, 1, 0, s>>>(dst, v);
+  return cudaGetLastError();
+}
 cudaError_t launch_aos_to_soa(const DevRun& r, const double* aos, double* soa, int* bad, cudaStream_t s) {
   const size_t n = (size_t)r.imax * r.jmax * r.kmax;
   k_aos_to_soa<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(r, aos, soa, bad);

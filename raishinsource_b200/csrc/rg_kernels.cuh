@@ -96,6 +96,8 @@ cudaError_t launch_rkt(const DevRun& r, int stage, const double* W1, const doubl
                        const double* Uo, const double* Uc, const double* SF, double* Unew, double dt, cudaStream_t s);
 // reference layout a(nv,i,j,k) of the full array <-> the run's stored SoA
 // (bad, if given, is set non-zero when the data are not uniform along a slab direction)
+// the run's scalar block
+cudaError_t launch_set_scal(Scal* dst, const Scal& v, cudaStream_t s);
 cudaError_t launch_aos_to_soa(const DevRun& r, const double* aos, double* soa, int* bad, cudaStream_t s);
 cudaError_t launch_soa_to_aos(const DevRun& r, const double* soa, double* aos, cudaStream_t s);
 cudaError_t launch_fill(double* p, double v, size_t n, cudaStream_t s);
