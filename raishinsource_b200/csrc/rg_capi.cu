@@ -104,7 +104,7 @@ struct rg_ctx {
   std::map<int, Run*> runs;
   std::map<std::vector<int>, BatchEntry*> batches;
   struct Tuned { int width, group, grid_factor; double ms; };
-  std::map<long long, Tuned> tuned;  // batch class -> shape chosen by the tuner and its step time
+  std::map<long long, Tuned> tuned;  // batch class and size (tune_class) -> shape chosen by the tuner and its step time
   int next_id = 1;
   long long launches[K_NKINDS] = {};   // kernel launches issued, per kind
   bool prof = false;                   // bracket every launch with CUDA events
@@ -722,6 +722,17 @@ long long batch_class(const Run* R) {
   return (long long)d.ict * 100000 + (long long)d.irec * 1000 + d.mixed * 100 + (d.jfix ? 10 : 0) + (d.kfix ? 1 : 0);
 }
 
+// Key of a tuned shape: the class and the batch's size in powers of two.  The
+// shape that suits one small torus (persistent grids of two blocks per SM are
+// as good as any there) takes 1.8 times as long on one sixteen times its size.
+long long tune_class(const std::vector<Run*>& rs) {
+  size_t cells = 0;
+  for (const Run* R : rs) cells += R->d.N;
+  int lg = 0;
+  while (cells >>= 1) ++lg;
+  return batch_class(rs[0]) * 64 + lg;
+}
+
 int kind_of(const BatchPlan* B, int idx) {
   int dir = 0;
   switch (batch_launch_kind(B, idx, &dir)) {
@@ -790,8 +801,7 @@ constexpr int kTuneAfter = 32;
 int make_batch(rg_ctx* ctx, std::vector<Run*>& rs, const std::vector<int>& ids, BatchEntry** out) {
   std::vector<DevRun> dr;
   for (Run* R : rs) dr.push_back(R->d);
-  const long long cls = batch_class(rs[0]);
-  auto tk = ctx->tuned.find(cls);
+  auto tk = ctx->tuned.find(tune_class(rs));
   BatchEntry* E = new BatchEntry();
   E->ids = ids;
   if (tk != ctx->tuned.end()) {
@@ -886,7 +896,7 @@ int tune_batch(rg_ctx* ctx, BatchEntry* E) {
   E->grid_factor = keep_factor;
   E->tuned_ms = best / 2.0;
   E->tune_pending = false;
-  ctx->tuned[batch_class(rs[0])] = {E->width, E->group, E->grid_factor, E->tuned_ms};
+  ctx->tuned[tune_class(rs)] = {E->width, E->group, E->grid_factor, E->tuned_ms};
   return capture_batch(E);
 }
 
