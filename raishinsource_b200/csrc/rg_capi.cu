@@ -113,6 +113,8 @@ struct rg_ctx {
   double ms[K_NKINDS] = {};
   bool own_stream = true;              // false after rg_ctx_set_stream
   cudaEvent_t marks[RG_MAX_MARKS] = {};  // rg_ctx_mark / rg_ctx_wait_mark
+  cudaStream_t side[2] = {nullptr, nullptr};  // the phi and theta faces of small 3D runs (run_stage)
+  cudaEvent_t fork[3] = {nullptr, nullptr, nullptr};
   int* flag = nullptr;                 // one word of pinned host memory that kernels write (uploaded data not uniform)
   bool tma = true;                     // staged face kernel where a run allows it (RAISHIN_FLUX_TMA=0: off)
   bool utma = true;                    // staged update kernel where a run allows it (RAISHIN_UPDATE_TMA=0: off)
@@ -640,6 +642,9 @@ int drain_events(rg_ctx* ctx) {
   return RG_OK;
 }
 
+// Stored cells below which a stage's three face kernels run side by side.
+constexpr long long kForkFaces = 1 << 18;
+
 // One RK3 stage (main.f90:807-911 / 919-1032 / 1043-1147).
 int run_stage(rg_ctx* ctx, Run* R, int stage, const double* Pn, const double* Pc, double* Pw) {
   const DevRun& d = R->d;
@@ -648,14 +653,29 @@ int run_stage(rg_ctx* ctx, Run* R, int stage, const double* Pn, const double* Pc
   // the faces with the stencil staged by TMA where the run allows it
   const int bi = (Pc == R->b.P[0]) ? 0 : (Pc == R->b.P[1] ? 1 : 2);
   const bool tma = R->tma && ctx->tma && Pc == R->b.P[bi];
-  auto faces = [&](int dir) {
+  auto faces = [&](int dir, cudaStream_t fs) {
     return tma ? launch_flux_tma(d, dir, &R->tmap[bi][dir - 1], &R->tmap32[dir - 1], &R->tmapm[dir - 1],
-                                 R->b.F[dir - 1], s)
-               : launch_flux(d, dir, Pc, R->b.F[dir - 1], s);
+                                 R->b.F[dir - 1], fs)
+               : launch_flux(d, dir, Pc, R->b.F[dir - 1], fs);
   };
-  RG_CUDA(issue(ctx, K_FLUX1, nf, [&] { return faces(1); }));
-  RG_CUDA(issue(ctx, K_FLUX2, nf, [&] { return faces(2); }));
-  RG_CUDA(issue(ctx, K_FLUX3, nf, [&] { return faces(3); }));
+  // The three directions read the same state and write arrays of their own.  On
+  // a grid whose faces of one direction fill the GPU less than about twice
+  // they run side by side (timed runs keep one kernel at a time).
+  const long long nface = (long long)d.imax * d.jpl * d.kpl;
+  if (ctx->prof || nface > kForkFaces) {
+    RG_CUDA(issue(ctx, K_FLUX1, nf, [&] { return faces(1, s); }));
+    RG_CUDA(issue(ctx, K_FLUX2, nf, [&] { return faces(2, s); }));
+    RG_CUDA(issue(ctx, K_FLUX3, nf, [&] { return faces(3, s); }));
+  } else {
+    RG_CUDA(cudaEventRecord(ctx->fork[0], s));
+    for (int a = 0; a < 2; ++a) {
+      RG_CUDA(cudaStreamWaitEvent(ctx->side[a], ctx->fork[0], 0));
+      RG_CUDA(issue(ctx, K_FLUX2 + a, nf, [&] { return faces(2 + a, ctx->side[a]); }));
+      RG_CUDA(cudaEventRecord(ctx->fork[1 + a], ctx->side[a]));
+    }
+    RG_CUDA(issue(ctx, K_FLUX1, nf, [&] { return faces(1, s); }));
+    for (int a = 0; a < 2; ++a) RG_CUDA(cudaStreamWaitEvent(s, ctx->fork[1 + a], 0));
+  }
   RG_CUDA(issue(ctx, K_CT, n_ct_launches(d), [&] { return launch_ct(d, Pc, R->b.F[0], R->b.F[1], R->b.F[2], R->b.CT, s); }));
   if (d.iwvec == 2) {
     const size_t N = d.N;
@@ -943,6 +963,10 @@ int rg_ctx_create(int device, rg_ctx** out) {
   if (const char* t = std::getenv("RAISHIN_UPDATE_TMA")) c->utma = std::strcmp(t, "0") != 0;
   cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&c->flag), sizeof(int), cudaHostAllocMapped);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+  for (cudaStream_t& t : c->side)
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking);
+  for (cudaEvent_t& t : c->fork)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     cudaFreeHost(c->flag);
     delete c;
@@ -963,6 +987,8 @@ int rg_ctx_destroy(rg_ctx* ctx) {
   for (cudaEvent_t e : ctx->marks)
     if (e) cudaEventDestroy(e);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
+  for (cudaStream_t t : ctx->side) cudaStreamDestroy(t);
+  for (cudaEvent_t t : ctx->fork) cudaEventDestroy(t);
   cudaFreeHost(ctx->flag);
   delete ctx;
   return RG_OK;
