@@ -115,7 +115,9 @@ struct rg_ctx {
   cudaEvent_t marks[RG_MAX_MARKS] = {};  // rg_ctx_mark / rg_ctx_wait_mark
   cudaStream_t side[2] = {nullptr, nullptr};  // the phi and theta faces of small 3D runs (run_stage)
   cudaEvent_t fork[3] = {nullptr, nullptr, nullptr};
-  int* flag = nullptr;                 // one word of pinned host memory that kernels write (uploaded data not uniform)
+  // pinned host memory that kernels write: one word (uploaded data not uniform), and from byte 64 the counters of
+  // rg_calflx_static, whose call must read them without a device copy
+  int* flag = nullptr;
   bool tma = true;                     // staged face kernel where a run allows it (RAISHIN_FLUX_TMA=0: off)
   bool utma = true;                    // staged update kernel where a run allows it (RAISHIN_UPDATE_TMA=0: off)
 };
@@ -158,6 +160,20 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
+// The tensor map of nv planes of the run's cells at base (eb bytes a value) as
+// the 4D array (i, j, k, v) with the given box.
+bool encode_planes(const DevRun& d, CUtensorMap* tm, void* base, int eb, int nv, const unsigned box[4]) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const cuuint64_t dims[4] = {(cuuint64_t)d.imax, (cuuint64_t)d.jmax, (cuuint64_t)d.kmax, (cuuint64_t)nv};
+  const cuuint64_t strides[3] = {(cuuint64_t)d.imax * eb, (cuuint64_t)d.imax * d.jmax * eb, (cuuint64_t)d.N * eb};
+  const cuuint32_t bx[4] = {box[0], box[1], box[2], box[3]};
+  return enc(tm, eb == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides,
+             bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Tensor maps of the three primitive buffers (and of P32 for a mixed run) as
 // 4D arrays (i, j, k, v) with the boxes of the staged face kernel, and of the
 // update's flux, flux-CT and U^n arrays with the boxes of the staged update;
@@ -171,12 +187,7 @@ void make_tmaps(Run* R) {
   if (!enc) return;
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   auto encode = [&](CUtensorMap* tm, void* base, int eb, int nv, const unsigned box[4]) {
-    const cuuint64_t dims[4] = {(cuuint64_t)d.imax, (cuuint64_t)d.jmax, (cuuint64_t)d.kmax, (cuuint64_t)nv};
-    const cuuint64_t strides[3] = {(cuuint64_t)d.imax * eb, (cuuint64_t)d.imax * d.jmax * eb, (cuuint64_t)d.N * eb};
-    const cuuint32_t bx[4] = {box[0], box[1], box[2], box[3]};
-    return enc(tm, eb == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims,
-               strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode_planes(d, tm, base, eb, nv, box);
   };
   if (flux_tma_eligible(d)) {
     bool ok = true;
@@ -961,7 +972,8 @@ int rg_ctx_create(int device, rg_ctx** out) {
   c->device = device;
   if (const char* t = std::getenv("RAISHIN_FLUX_TMA")) c->tma = std::strcmp(t, "0") != 0;
   if (const char* t = std::getenv("RAISHIN_UPDATE_TMA")) c->utma = std::strcmp(t, "0") != 0;
-  cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&c->flag), sizeof(int), cudaHostAllocMapped);
+  cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&c->flag), 64 + C_NCOUNTERS * sizeof(unsigned long long),
+                                cudaHostAllocMapped);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   for (cudaStream_t& t : c->side)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking);
@@ -2207,12 +2219,31 @@ extern "C" int rg_calflx_static(rg_ctx* ctx, int run, const double* d_prims, dou
   RG_CUDA(cudaMemsetAsync(ct, 0, 6 * N * sizeof(double), s));
   k_static_scal_reset<<<1, 1, 0, s>>>(d.scal);
   RG_CUDA(cudaGetLastError());
-  for (int dir = 1; dir <= 3; ++dir) RG_CUDA(launch_flux(d, dir, d_prims, d_ww + (size_t)(dir - 1) * 9 * N, s));
+  // The staged face kernel where the run's own steps take it (its face-metric
+  // maps exist then) and the caller's array starts on a 16-byte boundary, as
+  // the tensor maps, encoded here for each call's array, require.
+  CUtensorMap maps[3];
+  bool staged = R->tma && ctx->tma && flux_tma_eligible(d) && reinterpret_cast<uintptr_t>(d_prims) % 16 == 0;
+  for (int dir = 1; dir <= 3 && staged; ++dir) {
+    unsigned box[4];
+    flux_tma_box(dir, 8, d.irec, box);
+    staged = encode_planes(d, &maps[dir - 1], const_cast<double*>(d_prims), 8, 9, box);
+  }
+  unsigned long long* cnt = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(ctx->flag) + 64);
+  std::memset(cnt, 0, C_NCOUNTERS * sizeof(unsigned long long));
+  d.cnt = cnt;
+  for (int dir = 1; dir <= 3; ++dir) {
+    double* F = d_ww + (size_t)(dir - 1) * 9 * N;
+    if (staged) RG_CUDA(launch_flux_tma(d, dir, &maps[dir - 1], nullptr, &R->tmapm[dir - 1], F, s));
+    else RG_CUDA(launch_flux(d, dir, d_prims, F, s));
+  }
   RG_CUDA(launch_ct(d, d_prims, d_ww, d_ww + 9 * N, d_ww + 18 * N, ct, s));
   const dim3 b(64, 4, 1);
   const int n = d.imax - 2 * d.nm1 + 1, m = d.jmax - 2 * d.nm1 + 1, l = d.kmax - 2 * d.nm1 + 1;
   k_ct_scatter<<<dim3((n + 63) / 64, (m + 3) / 4, l), b, 0, s>>>(d, ct, d_ww);
   RG_CUDA(cudaGetLastError());
   RG_CUDA(cudaStreamSynchronize(s));
+  if (static_cast<volatile unsigned long long*>(cnt)[C_TMAWAIT])
+    return fail(RG_ECUDA, "a TMA wait of a staged face kernel ran out");
   return RG_OK;
 }
