@@ -223,7 +223,11 @@ void plan_append(BatchPlan& B, std::vector<Tile>& T, BLaunch L, const std::vecto
 // along i (64 or 128: the batched kernels are compiled for at most 128, the
 // CT kernel for 2 * 128) and `group` the blocks along i of one tile, so a
 // tile of a cell kernel covers width * group cells along i.
-int batch_build(const std::vector<DevRun>& runs, int width, int group, BatchPlan** out) {
+// The tables are copied on the stream whose launches read them: a copy on the
+// legacy default stream may still be on its way to the device when cudaMemcpy
+// returns (it waits for the staging of pageable memory only), and a
+// non-blocking stream does not wait for that stream.
+int batch_build(const std::vector<DevRun>& runs, int width, int group, cudaStream_t s, BatchPlan** out) {
   if (width != 64 && width != 128) return 1;
   if (group < 1) group = 1;
   BatchPlan* B = new BatchPlan();
@@ -363,8 +367,8 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, BatchPlan
     delete B;
     return 1;
   }
-  if (cudaMemcpy(B->d_runs, runs.data(), runs.size() * sizeof(DevRun), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(B->d_tiles, T.data(), T.size() * sizeof(Tile), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemcpyAsync(B->d_runs, runs.data(), runs.size() * sizeof(DevRun), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+      cudaMemcpyAsync(B->d_tiles, T.data(), T.size() * sizeof(Tile), cudaMemcpyHostToDevice, s) != cudaSuccess) {
     cudaFree(B->d_runs);
     cudaFree(B->d_tiles);
     delete B;

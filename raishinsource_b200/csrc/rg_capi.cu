@@ -843,7 +843,7 @@ int make_batch(rg_ctx* ctx, std::vector<Run*>& rs, const std::vector<int>& ids, 
   } else {
     E->tune_pending = true;
   }
-  if (batch_build(dr, E->width, E->group, &E->plan)) {
+  if (batch_build(dr, E->width, E->group, ctx->stream, &E->plan)) {
     delete E;
     return fail(RG_ENOMEM_ADMIT, "batch tables do not fit");
   }
@@ -884,7 +884,7 @@ int tune_batch(rg_ctx* ctx, BatchEntry* E) {
   int keep_factor = E->grid_factor;
   for (const Shape& sh : shapes) {
     BatchPlan* P = nullptr;
-    if (batch_build(dr, sh.width, sh.group, &P)) return fail(RG_ENOMEM_ADMIT, "batch tables do not fit");
+    if (batch_build(dr, sh.width, sh.group, s, &P)) return fail(RG_ENOMEM_ADMIT, "batch tables do not fit");
     for (int f : factors) {
       batch_set_grid(P, f);
       float ms = 0.f;
@@ -916,7 +916,7 @@ int tune_batch(rg_ctx* ctx, BatchEntry* E) {
   cudaEventDestroy(e1);
   RG_CUDA(cudaStreamSynchronize(s));
   BatchPlan* P = nullptr;
-  if (batch_build(dr, keep.width, keep.group, &P)) return fail(RG_ENOMEM_ADMIT, "batch tables do not fit");
+  if (batch_build(dr, keep.width, keep.group, s, &P)) return fail(RG_ENOMEM_ADMIT, "batch tables do not fit");
   batch_set_grid(P, keep_factor);
   if (E->graph) cudaGraphExecDestroy(E->graph);
   E->graph = nullptr;

@@ -123,7 +123,7 @@ cudaError_t launch_ic_torus(const DevRun& r, const IcTorusArgs& a, double* P, cu
 
 // Batched steps of runs of one class (rg_batch.cuh).
 struct BatchPlan;
-int batch_build(const std::vector<DevRun>& runs, int width, int group, BatchPlan** out);
+int batch_build(const std::vector<DevRun>& runs, int width, int group, cudaStream_t s, BatchPlan** out);
 void batch_destroy(BatchPlan* B);
 int batch_launch_count(const BatchPlan* B);
 void batch_set_grid(BatchPlan* B, int factor);
