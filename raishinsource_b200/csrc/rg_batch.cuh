@@ -104,21 +104,14 @@ struct UpdateB {
   }
 };
 
-template <int STAGE>
-struct CarryB {
-  __device__ void operator()(const DevRun& r, const Tile&) const {
-    double *Pn, *Pc, *Pw;
-    stage_ptrs(r, STAGE, Pn, Pc, Pw);
-    carry_fix_body<0, STAGE>(r, Pn, Pc, Pw, r.F[0], r.F[1], r.F[2], r.CT, nullptr);
-  }
-};
-
+// The straggler pass and, after a run's last tile of it, the W carry (t.aux: the run's tiles).
 template <int STAGE>
 struct StragB {
   __device__ void operator()(const DevRun& r, const Tile& t) const {
     double *Pn, *Pc, *Pw;
     stage_ptrs(r, STAGE, Pn, Pc, Pw);
     straggler_body<STAGE>(r, Pn, Pc, Pw, r.F[0], r.F[1], r.F[2], r.CT, make_uint3(t.bx, 0, 0));
+    if (last_block(r, t.aux)) carry_fix_body<0, STAGE>(r, Pn, Pc, Pw, r.F[0], r.F[1], r.F[2], r.CT, nullptr);
   }
 };
 
@@ -131,6 +124,15 @@ struct BcB {
     // one variable per z index of the grid, as the single-run passes take it
     if (PERIODIC) bc_periodic_body<D>(r, Pw, make_uint3(t.bx, t.by, 0), t.bz, t.bz + 1);
     else bc_phys_body<D>(r, Pw, Pn, make_uint3(t.bx, t.by, 0), t.bz, t.bz + 1);
+  }
+};
+
+struct BcAllB {
+  int stage;
+  __device__ void operator()(const DevRun& r, const Tile& t) const {
+    double *Pn, *Pc, *Pw;
+    stage_ptrs(r, stage, Pn, Pc, Pw);
+    bc_all_body(r, Pw, make_uint3(t.bx, t.by, t.bz));
   }
 };
 
@@ -167,7 +169,7 @@ struct ScalarB {
 // ------------------------------------------------------------- host side
 // One launch of a batched step: the kernel to run and its tile range.
 enum BKind {
-  BK_BEGIN, BK_CFL, BK_DT, BK_FLUX, BK_CT, BK_UPDATE, BK_CARRY, BK_BCPER, BK_BCPHYS, BK_FLOOR, BK_END, BK_STRAG
+  BK_BEGIN, BK_CFL, BK_DT, BK_FLUX, BK_CT, BK_UPDATE, BK_BCALL, BK_BCPER, BK_BCPHYS, BK_FLOOR, BK_END, BK_STRAG
 };
 struct BLaunch {
   int kind;
@@ -241,7 +243,8 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, cudaStrea
   cudaDeviceGetAttribute(&B->sm_count, cudaDevAttrMultiProcessorCount, dev);
   std::vector<Tile> T;
   const DevRun& r0 = runs[0];
-  const bool mixed = r0.mixed != 0;
+  bool one_pass = true;  // the ghosts of every member in one pass
+  for (const DevRun& r : runs) one_pass = one_pass && bc_one_pass(r);
   auto one = [](int a, const DevRun&, std::vector<Tile>& t) { add_tiles(t, a, dim3(1, 1, 1), 0, 0, 0); };
   BLaunch L{};
   L.block = dim3(32, 1, 1);
@@ -320,12 +323,18 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, cudaStrea
     L.kind = BK_STRAG;
     L.block = dim3(128, 1, 1);
     plan_append(*B, T, L, runs, [&](int a, const DevRun& r, std::vector<Tile>& t) {
-      if (r.strag_list) add_tiles(t, a, dim3((unsigned)((r.strag_cap + 127) / 128), 1, 1), 0, 0, 0);
+      const int n = (r.strag_cap + 127) / 128;
+      add_tiles(t, a, dim3((unsigned)n, 1, 1), 0, 0, n);
     });
-    L.kind = BK_CARRY;
-    L.block = dim3(128, 1, 1);
-    plan_append(*B, T, L, runs, one);
-    for (int per = 1; per >= 0; --per)
+    if (one_pass) {
+      L.kind = BK_BCALL;
+      L.dir = 0;
+      L.block = dim3(128, 1, 1);
+      plan_append(*B, T, L, runs, [&](int a, const DevRun& r, std::vector<Tile>& t) {
+        add_tiles(t, a, dim3(bc_all_blocks(r), 1, 1), 0, 0, 0);
+      });
+    }
+    for (int per = one_pass ? -1 : 1; per >= 0; --per)
       for (int dir = 1; dir <= 3; ++dir) {
         L.kind = per ? BK_BCPER : BK_BCPHYS;
         L.dir = dir;
@@ -360,7 +369,6 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, cudaStrea
   L.kind = BK_END;
   L.block = dim3(32, 1, 1);
   plan_append(*B, T, L, runs, one);
-  (void)mixed;
   if (cudaMalloc(&B->d_runs, runs.size() * sizeof(DevRun)) != cudaSuccess ||
       cudaMalloc(&B->d_tiles, T.size() * sizeof(Tile)) != cudaSuccess) {
     cudaFree(B->d_runs);
@@ -476,10 +484,7 @@ cudaError_t batch_issue(const BatchPlan* B, int idx, cudaStream_t s) {
       if (L.stage == 1) return kb_go<StragB<1>, 128, 1>(B, L, StragB<1>{}, s);
       if (L.stage == 2) return kb_go<StragB<2>, 128, 1>(B, L, StragB<2>{}, s);
       return kb_go<StragB<3>, 128, 1>(B, L, StragB<3>{}, s);
-    case BK_CARRY:
-      if (L.stage == 1) return kb_go<CarryB<1>, 128, 1>(B, L, CarryB<1>{}, s);
-      if (L.stage == 2) return kb_go<CarryB<2>, 128, 1>(B, L, CarryB<2>{}, s);
-      return kb_go<CarryB<3>, 128, 1>(B, L, CarryB<3>{}, s);
+    case BK_BCALL: return kb_go<BcAllB, 128, 1>(B, L, BcAllB{L.stage}, s);
     case BK_BCPER:
     case BK_BCPHYS:
       if (L.dir == 1) return go_bc<1>(B, L, s);

@@ -770,8 +770,8 @@ int kind_of(const BatchPlan* B, int idx) {
     case 1: return K_CFL;
     case 3: return K_FLUX1;  // one launch for the faces of all directions
     case 4: return K_CT;
-    case 5: case 6: return K_UPDATE;
-    case 7: case 8: return K_BC;
+    case 5: return K_UPDATE;
+    case 6: case 7: case 8: return K_BC;
     case 9: return K_FLOOR;
     case 11: return K_UPDATE;
     default: return K_SCALAR;

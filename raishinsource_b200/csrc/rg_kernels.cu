@@ -773,7 +773,7 @@ __device__ __forceinline__ bool queue_straggler(const DevRun& r, int i, int j, i
 #endif
 
 // recov1a of one interior cell from its stage conserved state u, with
-// straggler deferral (the cell is queued for k_straggler when its iteration
+// straggler deferral (the cell is queued for the straggler pass when its iteration
 // count passes kDeferIter and the list has room) and the loop-order W carry
 // for cells without a root; the primitives go to Pw.
 __device__ __forceinline__ void update_recov(const DevRun& r, int i, int j, int k, const Met& m,
@@ -865,13 +865,22 @@ __device__ __forceinline__ void straggler_body(const DevRun& r, const double* __
   count_event(r, C_CAP, ok && o.cap);
 }
 
-template <int STAGE>
-__global__ void __launch_bounds__(128) k_straggler(DevRun r, const double* __restrict__ Pn,
-                                                   const double* __restrict__ Pc, double* __restrict__ Pw,
-                                                   const double* __restrict__ F1, const double* __restrict__ F2,
-                                                   const double* __restrict__ F3, const double* __restrict__ CT) {
-  straggler_body<STAGE>(r, Pn, Pc, Pw, F1, F2, F3, CT, blockIdx);
+// The last of a run's `parts` blocks of a pass to get here: true in every thread
+// of that block, which sees what the others wrote.
+__device__ __forceinline__ bool last_block(const DevRun& r, int parts) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
+    last = atomicAdd(&r.scal->ticket, 1) == parts - 1;
+    if (last) r.scal->ticket = 0;
+  }
+  __syncthreads();
+  const bool l = last != 0;
+  if (l) __threadfence();
+  return l;
 }
+
 template <int STAGE, bool MIX>
 __global__ void __launch_bounds__(128, RG_UPDATE_MINB) k_update(DevRun r, const double* __restrict__ Pn, const double* __restrict__ Pc,
                                                 double* __restrict__ Pw, const double* __restrict__ F1,
@@ -963,6 +972,19 @@ __global__ void __launch_bounds__(kCarryThreads) k_carry_fix(DevRun r, const dou
   // one block: every thread takes part (the body ranks the queued cells and
   // runs the chains with the whole block, with block barriers)
   carry_fix_body<MODE, STAGE, IWVEC>(r, Pn, Pc, Pw, F1, F2, F3, CT, U);
+}
+
+// The straggler pass, and after its last block the loop-order W carry: both
+// are idle in most stages, and one launch of an idle pass costs what two do.
+template <int STAGE>
+__global__ void __launch_bounds__(kCarryThreads) k_strag_carry(DevRun r, const double* __restrict__ Pn,
+                                                               const double* __restrict__ Pc, double* __restrict__ Pw,
+                                                               const double* __restrict__ F1,
+                                                               const double* __restrict__ F2,
+                                                               const double* __restrict__ F3,
+                                                               const double* __restrict__ CT) {
+  straggler_body<STAGE>(r, Pn, Pc, Pw, F1, F2, F3, CT, blockIdx);
+  if (last_block(r, (int)gridDim.x)) carry_fix_body<0, STAGE>(r, Pn, Pc, Pw, F1, F2, F3, CT, nullptr);
 }
 
 // ------------------------------------------------------------- face fluxes
@@ -2114,6 +2136,88 @@ __global__ void k_bc_phys(DevRun r, double* __restrict__ P, const double* __rest
   bc_phys_body<D>(r, P, Po, blockIdx, (int)blockIdx.z, (int)blockIdx.z + 1);
 }
 
+// All ghost cells in one pass.  Where every code copies, mirrors, zeroes or
+// wraps an interior cell (bc_one_pass), the passes in the reference's order
+// compose to one interior source per ghost cell and variable: the theta pass
+// ran last, on every column, so a theta ghost is the mirror of a cell of its
+// own column, which, if it is a radial ghost, came from a cell of its row,
+// which, if it is a phi ghost, came from its period.  Sources are interior
+// cells, which no thread writes.  Three launches of dependent chains become
+// one; the values are the same copies.
+__device__ __forceinline__ int mirror_src(int code, int n, int L, int nm1, double& sign) {
+  if (code == 5) return n <= nm1 ? 1 + nm1 : L - nm1;
+  if (code == 13) sign = 0.0;
+  if (code == 12) sign = -sign;
+  return n <= nm1 ? 2 * nm1 - n + 1 : 2 * L - 2 * nm1 + 1 - n;
+}
+// The ghost cells, numbered: theta ghosts (whole planes), then phi ghosts of the
+// interior theta rows, then radial ghosts of the interior columns; i fastest.
+// (A thread per cell of the whole grid, most of them leaving at once, took 0.17
+// ms a step on 256x128x128; the shell alone 0.095, the three passes 0.132.)
+RG_HD inline void ghost_counts(const DevRun& r, unsigned n[3]) {
+  const unsigned g = 2u * (unsigned)r.nm1, I = (unsigned)r.imax, J = r.jfix ? 1u : (unsigned)r.jmax;
+  const unsigned ki = r.kfix ? 1u : (unsigned)r.kmax - g, ji = r.jfix ? 1u : J - g;
+  n[0] = r.kfix ? 0u : I * J * g;
+  n[1] = r.jfix ? 0u : I * g * ki;
+  n[2] = g * ji * ki;
+}
+__device__ __forceinline__ void bc_all_body(const DevRun& r, double* __restrict__ P, const uint3 bid) {
+  if (!r.scal->active) return;
+  unsigned t = bid.x * blockDim.x + threadIdx.x, cnt[3];
+  ghost_counts(r, cnt);
+  const int nm1 = r.nm1;
+  const unsigned g = 2u * (unsigned)nm1, I = (unsigned)r.imax, J = r.jfix ? 1u : (unsigned)r.jmax;
+  // n-th ghost index of a direction of L cells; n-th interior index (a slab's own index)
+  auto ghost = [&](unsigned n, int L) { return (int)n < nm1 ? (int)n + 1 : L - 2 * nm1 + (int)n + 1; };
+  int i, j, k;
+  if (t < cnt[0]) {
+    i = (int)(t % I) + 1;
+    t /= I;
+    j = r.jfix ? r.jfix : (int)(t % J) + 1;
+    k = ghost(t / J, r.kmax);
+  } else if ((t -= cnt[0]) < cnt[1]) {
+    i = (int)(t % I) + 1;
+    t /= I;
+    j = ghost(t % g, r.jmax);
+    k = r.kfix ? r.kfix : (int)(t / g) + nm1 + 1;
+  } else if ((t -= cnt[1]) < cnt[2]) {
+    i = ghost(t % g, r.imax);
+    t /= g;
+    const unsigned ji = r.jfix ? 1u : J - g;
+    j = r.jfix ? r.jfix : (int)(t % ji) + nm1 + 1;
+    k = r.kfix ? r.kfix : (int)(t / ji) + nm1 + 1;
+  } else {
+    return;
+  }
+  const bool gi = i <= nm1 || i > r.imax - nm1;
+  const bool gj = !r.jfix && (j <= nm1 || j > r.jmax - nm1);
+  const bool gk = !r.kfix && (k <= nm1 || k > r.kmax - nm1);
+  const size_t N = r.N, c = r.cell(i, j, k);
+  const int period = r.jmax - 2 * nm1;
+  const int sj = gj ? (j <= nm1 ? j + period : j - period) : j;
+  double val[9];
+#pragma unroll
+  for (int v = 0; v < 9; ++v) {
+    double sign = 1.0;
+    int si = i, sk = k;
+    if (gk) sk = mirror_src(r.ibc[k <= nm1 ? 4 : 5][v], k, r.kmax, nm1, sign);
+    if (gi) {
+      const int code = r.ibc[i <= nm1 ? 0 : 1][v];
+      if (code == 18) {  // x1 outer (bnd.f90:598-610): zero when u^r of the last interior cell is negative
+        si = r.imax - nm1;
+        if (P[N + r.cell(si, sj, sk)] < 0.0) sign = 0.0;
+      } else {
+        si = mirror_src(code, i, r.imax, nm1, sign);
+      }
+    }
+    const double x = P[(size_t)v * N + r.cell(si, sj, sk)];
+    val[v] = sign == 1.0 ? x : (sign == 0.0 ? 0.0 : -x);
+  }
+#pragma unroll
+  for (int v = 0; v < 9; ++v) P[(size_t)v * N + c] = val[v];
+}
+__global__ void __launch_bounds__(128) k_bc_all(DevRun r, double* __restrict__ P) { bc_all_body(r, P, blockIdx); }
+
 // ----------------------------------------------------------------- floors
 // infchk (bnd.f90:1636-1824, outer radial ghosts), atmosphere1a
 // (correction.f90:226-447) and pminmax2b (correction.f90:744-999) over every
@@ -2980,15 +3084,10 @@ cudaError_t launch_update(const DevRun& r, int stage, const double* Pn, const do
       launch_update_t<true>(r, stage, Pn, Pc, Pw, F1, F2, F3, CT, split + 1, r.imax, s);
     }
   }
-  if (r.strag_list) {
-    const unsigned gs = (unsigned)((r.strag_cap + 127) / 128);
-    if (stage == 1) k_straggler<1><<<gs, 128, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT);
-    else if (stage == 2) k_straggler<2><<<gs, 128, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT);
-    else k_straggler<3><<<gs, 128, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT);
-  }
-  if (stage == 1) k_carry_fix<0, 1><<<1, kCarryThreads, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT, nullptr);
-  else if (stage == 2) k_carry_fix<0, 2><<<1, kCarryThreads, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT, nullptr);
-  else k_carry_fix<0, 3><<<1, kCarryThreads, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT, nullptr);
+  const unsigned gs = (unsigned)((r.strag_cap + kCarryThreads - 1) / kCarryThreads);
+  if (stage == 1) k_strag_carry<1><<<gs, kCarryThreads, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT);
+  else if (stage == 2) k_strag_carry<2><<<gs, kCarryThreads, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT);
+  else k_strag_carry<3><<<gs, kCarryThreads, 0, s>>>(r, Pn, Pc, Pw, F1, F2, F3, CT);
   return cudaGetLastError();
 }
 
@@ -3005,7 +3104,7 @@ int n_ct_launches(const DevRun& r) {
   return (split >= lo) + (split < hi);
 }
 int n_update_launches(const DevRun& r) {
-  const int extra = 1 + (r.strag_list ? 1 : 0);  // carry fix, straggler pass
+  const int extra = 1;  // straggler pass and carry fix
   if (!r.mixed) return 1 + extra;
   const int split = fp64_split(r, 1, r.imax);
   return (split >= 1) + (split < r.imax) + extra;
@@ -3036,7 +3135,32 @@ static void bc_shape9(int n1, int n2, bool fix1, bool fix2, dim3& g, dim3& b) {
   g.z = 9;
 }
 
+// Whether one pass fills the ghosts (bc_all_body): r and theta with codes that
+// copy, mirror or zero (5, 12, 13, 14; 18 at the outer r), phi periodic or a
+// slab, and at least nm1 interior cells along every stored direction, so
+// that every source is interior.
+static bool bc_one_pass(const DevRun& r) {
+  const int nm1 = r.nm1;
+  if (r.imax < 3 * nm1 || (!r.jfix && r.jmax < 3 * nm1) || (!r.kfix && r.kmax < 3 * nm1)) return false;
+  for (int v = 0; v < 9; ++v) {
+    for (int sd = 0; sd < 6; ++sd) {
+      const int c = r.ibc[sd][v];
+      const bool slab = (sd / 2 == 1 && r.jfix) || (sd / 2 == 2 && r.kfix);  // its own ghost fill is a no-op
+      const bool ok = slab || (sd / 2 == 1 ? c == 1 : (c == 5 || c == 12 || c == 13 || c == 14 || (c == 18 && sd == 1)));
+      if (!ok) return false;
+    }
+  }
+  return true;
+}
+
+static unsigned bc_all_blocks(const DevRun& r) {
+  unsigned n[3];
+  ghost_counts(r, n);
+  return (n[0] + n[1] + n[2] + 127u) / 128u;
+}
+
 int n_bc_launches(const DevRun& r) {
+  if (bc_one_pass(r)) return 1;
   int n = 0;
   for (int d = 0; d < 3; ++d) {
     const bool slab = (d == 1 && r.jfix) || (d == 2 && r.kfix);  // ghost fill of a slab plane is a no-op
@@ -3047,6 +3171,10 @@ int n_bc_launches(const DevRun& r) {
 }
 
 cudaError_t launch_bc(const DevRun& r, double* P, const double* Po, cudaStream_t s) {
+  if (bc_one_pass(r)) {
+    k_bc_all<<<bc_all_blocks(r), 128, 0, s>>>(r, P);
+    return cudaGetLastError();
+  }
   const int nm1 = r.nm1;
   const bool jf = r.jfix != 0, kf = r.kfix != 0;
   dim3 g, b;

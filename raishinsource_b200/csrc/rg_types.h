@@ -38,6 +38,7 @@ struct Scal {
   int carry_count;                // cells queued for the loop-order W carry fix-up
   int cur;                        // index of P^n among the run's three primitive buffers
   int strag_count;                // cells whose primitive recovery was deferred this stage
+  int ticket;                     // blocks of the straggler pass that have finished (0 between passes)
 };
 
 // Counters (device, atomically accumulated).
