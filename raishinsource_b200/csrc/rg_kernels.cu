@@ -59,10 +59,12 @@ constexpr int kRescaleCap = 1000;  // the reference's "go to 95" loop (recov.f90
 // primitives.  Returns false, touching nothing, when the W quadratic has no
 // non-negative root and no carried-in W is given: the reference then keeps W
 // from the previous cell of its loop (recov.f90:810-815), which the caller
-// resolves in loop order.
+// resolves in loop order.  need_s false: uri(6) is returned as 0 (the caller's
+// next pass, atmosphere1a, sets it to 0 in every cell: a cube root and a
+// division a cell).
 __device__ bool recov_cell(const double u[9], const double q[9], double out[9], const Met& m, double gam, int gkind,
                            int iter, double demin_i, double prmin_i, const double* wg_carry, RecovOut& res,
-                           int defer = 0x7fffffff) {
+                           int defer = 0x7fffffff, bool need_s = true) {
   const double safty = 1.0e-4, saftybig = 1.0e5, dv = 1.0e-2;
   const double gam1 = gam / (gam - 1.0), gam2 = 1.0 / gam1;
   const double idetg1 = m.idetg;  // 1. / detg1
@@ -289,10 +291,10 @@ __device__ bool recov_cell(const double u[9], const double q[9], double out[9], 
   // recov.f90:1174-1216 (the uu(6) rewrite is overwritten by caluu1 and is not kept)
   if (irecov == 0) {
     out[0] = ro; out[1] = util[1]; out[2] = util[2]; out[3] = util[3]; out[4] = pp;
-    out[5] = ro * pp / pow_gam1(ro, gam, gkind);
+    out[5] = need_s ? ro * pp / pow_gam1(ro, gam, gkind) : 0.0;
   } else {
     out[0] = q[0]; out[1] = q[1]; out[2] = q[2]; out[3] = q[3]; out[4] = q[4];
-    out[5] = q[0] * q[4] / pow_gam(q[0], gam, gkind);
+    out[5] = need_s ? q[0] * q[4] / pow_gam(q[0], gam, gkind) : 0.0;
   }
   out[6] = u[6] * idetg1;
   out[7] = u[7] * idetg1;
@@ -772,6 +774,9 @@ __device__ __forceinline__ bool queue_straggler(const DevRun& r, int i, int j, i
 #define RG_UPDATE_BX 32
 #endif
 
+// atmosphere1a runs for these models and sets uri(6) = 0 in every cell.
+__device__ __forceinline__ bool sets_s_zero(const DevRun& r) { return r.model >= 7 && r.model <= 15; }
+
 // recov1a of one interior cell from its stage conserved state u, with
 // straggler deferral (the cell is queued for the straggler pass when its iteration
 // count passes kDeferIter and the list has room) and the loop-order W carry
@@ -784,11 +789,13 @@ __device__ __forceinline__ void update_recov(const DevRun& r, int i, int j, int 
   load9(Pc, N, c, qo);
   RecovOut o{0.0, false, false, false};
   const double dei = __ldg(r.fl_de + i - 1), pri = __ldg(r.fl_pr + i - 1);
-  bool ok = recov_cell(u, qo, qn, m, r.gam, r.gkind, r.iter, dei, pri, nullptr, o, r.strag_list ? kDeferIter : 0x7fffffff);
+  const bool need_s = !sets_s_zero(r);
+  bool ok = recov_cell(u, qo, qn, m, r.gam, r.gkind, r.iter, dei, pri, nullptr, o,
+                       r.strag_list ? kDeferIter : 0x7fffffff, need_s);
   if (o.deferred) {
     if (queue_straggler(r, i, j, k)) return;
     o = RecovOut{0.0, false, false, false};
-    ok = recov_cell(u, qo, qn, m, r.gam, r.gkind, r.iter, dei, pri, nullptr, o);
+    ok = recov_cell(u, qo, qn, m, r.gam, r.gkind, r.iter, dei, pri, nullptr, o, 0x7fffffff, need_s);
   }
   if (!ok) {
     queue_carry(r, i, j, k);
@@ -2237,7 +2244,6 @@ __device__ __forceinline__ void floor_body(const DevRun& r, double* __restrict__
   load9(P, N, c, q);
   Met m;
   load_met(r.mc, r.nik, r.ik(i, k), m);
-  const double gam = r.gam;
   if ((PARTS & 1) && r.model >= 7 && r.model <= 20 && i > r.imax - r.nm1) {
     const double gflmax = 10.0;
     double gfl = calgfl(q[1], q[2], q[3], m);
@@ -2250,7 +2256,7 @@ __device__ __forceinline__ void floor_body(const DevRun& r, double* __restrict__
       q[1] = vel[1] * gfl; q[2] = vel[2] * gfl; q[3] = vel[3] * gfl;
     }
   }
-  if ((PARTS & 2) && r.model >= 7 && r.model <= 15) {
+  if ((PARTS & 2) && sets_s_zero(r)) {
     const double epsilon = 1.e-2, gflmax = 10.0;
     const double demin = __ldg(r.fl_de + i - 1);
     const double prmin = __ldg(r.fl_pr + i - 1);
