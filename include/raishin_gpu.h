@@ -186,8 +186,8 @@ int rg_run_stats(rg_ctx* ctx, int run, rg_step_stats* stats);
  * slab direction (3D runs, which fill the GPU alone) and runs with upwind
  * flux-CT or recov2 take each step with their own launches, after the
  * batches of that step, exactly as rg_step steps them.  The launch shape (block width, cells per tile
- * along i, persistent grid size) is tuned per batch class and context: a new
- * class starts with a default shape and, at the first segment boundary after
+ * along i, persistent grid size) is tuned per batch class, size (in powers of
+ * two) and context: a new one starts with a default shape and, at the first segment boundary after
  * 32 steps of its batch, times every candidate shape on trial steps from a
  * snapshot of the runs' state (which it restores) and keeps the fastest.
  * Each run's result equals its result stepped alone.  stats, if given,
@@ -206,7 +206,8 @@ int rg_batch_info(rg_ctx* ctx, const int* runs, int nruns, int* width, int* grid
  * rg_profile_read returns accumulated milliseconds and launch counts per kind:
  * 0 cfl, 1 flux r, 2 flux phi, 3 flux theta, 4 flux-CT, 5 update (+ W carry),
  * 6 ghost fill, 7 floors, 8 scalar bookkeeping.  Launch counts are kept with
- * profiling off too.  No counterpart in the reference (cpu_time only). */
+ * profiling off too.  The faces of a batched step (one launch for the three
+ * directions) count as kind 1.  No counterpart in the reference (cpu_time only). */
 int rg_profile(rg_ctx* ctx, int enable);
 int rg_profile_read(rg_ctx* ctx, double* ms, long long* launches, int nkinds);
 

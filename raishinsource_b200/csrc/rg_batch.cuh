@@ -153,14 +153,9 @@ struct CflB {
   }
 };
 
-// kind 0 step_begin, 1 dt, 2 step_end
-template <int KIND>
-struct ScalarB {
+struct EndB {
   __device__ void operator()(const DevRun& r, const Tile&) const {
-    if (threadIdx.x != 0) return;
-    if (KIND == 0) step_begin_body(r);
-    else if (KIND == 1) dt_body(r);
-    else step_end_body(r);
+    if (threadIdx.x == 0) step_end_body(r);
   }
 };
 
@@ -169,7 +164,7 @@ struct ScalarB {
 // ------------------------------------------------------------- host side
 // One launch of a batched step: the kernel to run and its tile range.
 enum BKind {
-  BK_BEGIN, BK_CFL, BK_DT, BK_FLUX, BK_CT, BK_UPDATE, BK_BCALL, BK_BCPER, BK_BCPHYS, BK_FLOOR, BK_END, BK_STRAG
+  BK_CFL, BK_FLUX, BK_CT, BK_UPDATE, BK_BCALL, BK_BCPER, BK_BCPHYS, BK_FLOOR, BK_END, BK_STRAG
 };
 struct BLaunch {
   int kind;
@@ -247,17 +242,11 @@ int batch_build(const std::vector<DevRun>& runs, int width, int group, cudaStrea
   for (const DevRun& r : runs) one_pass = one_pass && bc_one_pass(r);
   auto one = [](int a, const DevRun&, std::vector<Tile>& t) { add_tiles(t, a, dim3(1, 1, 1), 0, 0, 0); };
   BLaunch L{};
-  L.block = dim3(32, 1, 1);
-  L.kind = BK_BEGIN;
-  plan_append(*B, T, L, runs, one);
   L.kind = BK_CFL;
   L.block = wblock(r0, dim3(64, 2, 1), width);
   plan_append(*B, T, L, runs, [&](int a, const DevRun& r, std::vector<Tile>& t) {
     add_tiles(t, a, sgrid(r, r.imax - 2, r.jmax - 2, r.kmax - 2, L.block), 0, 0, 0, group);
   });
-  L.kind = BK_DT;
-  L.block = dim3(32, 1, 1);
-  plan_append(*B, T, L, runs, one);
   for (int stage = 1; stage <= 3; ++stage) {
     L.stage = stage;
     L.kind = BK_FLUX;
@@ -464,9 +453,7 @@ cudaError_t go_cell(const BatchPlan* B, const BLaunch& L, Body b, cudaStream_t s
 cudaError_t batch_issue(const BatchPlan* B, int idx, cudaStream_t s) {
   const BLaunch& L = B->launches[idx];
   switch (L.kind) {
-    case BK_BEGIN: return kb_go<ScalarB<0>, 32, 1>(B, L, ScalarB<0>{}, s);
-    case BK_DT: return kb_go<ScalarB<1>, 32, 1>(B, L, ScalarB<1>{}, s);
-    case BK_END: return kb_go<ScalarB<2>, 32, 1>(B, L, ScalarB<2>{}, s);
+    case BK_END: return kb_go<EndB, 32, 1>(B, L, EndB{}, s);
     case BK_CFL: return go_cell(B, L, CflB{}, s);
     case BK_FLUX:
       return L.fp32 ? go_flux_irec<float, float>(B, L, s) : go_flux_irec<double, double>(B, L, s);

@@ -516,11 +516,13 @@ std::vector<double> stored_from_full(const DevRun& d, const std::vector<double>&
 
 int set_time(rg_ctx* ctx, Run* R, double t0) {
   Scal s{};
-  s.dtcfl_bits = 0;
+  // the first step's loop top (step_begin_body)
+  const double one = 1.0;
+  std::memcpy(&s.dtcfl_bits, &one, sizeof(double));
   s.dt = 0.01;  // main.f90:358
   s.time = t0;
   s.timeh = t0;
-  s.active = 1;
+  s.active = !(t0 > R->d.tmax);
   s.carry_count = 0;
   RG_CUDA(launch_set_scal(R->d.scal, s, ctx->stream));
   return RG_OK;
@@ -767,13 +769,12 @@ long long tune_class(const std::vector<Run*>& rs) {
 int kind_of(const BatchPlan* B, int idx) {
   int dir = 0;
   switch (batch_launch_kind(B, idx, &dir)) {
-    case 1: return K_CFL;
-    case 3: return K_FLUX1;  // one launch for the faces of all directions
-    case 4: return K_CT;
-    case 5: return K_UPDATE;
-    case 6: case 7: case 8: return K_BC;
-    case 9: return K_FLOOR;
-    case 11: return K_UPDATE;
+    case 0: return K_CFL;
+    case 1: return K_FLUX1;  // one launch for the faces of all directions
+    case 2: return K_CT;
+    case 3: case 9: return K_UPDATE;
+    case 4: case 5: case 6: return K_BC;
+    case 7: return K_FLOOR;
     default: return K_SCALAR;
   }
 }
@@ -1395,9 +1396,7 @@ static int step_alone(rg_ctx* ctx, Run* R) {
   double* Pn = R->b.P[R->cur];
   double* P1 = R->b.P[(R->cur + 1) % 3];
   double* P2 = R->b.P[(R->cur + 2) % 3];
-  RG_CUDA(issue(ctx, K_SCALAR, 1, [&] { return launch_step_begin(R->d, s); }));
   RG_CUDA(issue(ctx, K_CFL, 1, [&] { return launch_cfl(R->d, Pn, s); }));
-  RG_CUDA(issue(ctx, K_SCALAR, 1, [&] { return launch_dt(R->d, s); }));
   int rc;
   if ((rc = run_stage(ctx, R, 1, Pn, Pn, P1))) return rc;
   if ((rc = run_stage(ctx, R, 2, Pn, P1, P2))) return rc;

@@ -7,7 +7,7 @@
 //             k_carry_fix   loop-order W carry of recov1a (only when queued)
 //             k_bc_*        ghost fill in the reference's pass order
 //             k_floor       infchk + atmosphere1a + pminmax2b (pointwise)
-// Per step:   k_step_begin, k_cfl (block min + atomicMin), k_dt, k_step_end.
+// Per step:   k_cfl (block min + atomicMin), k_step_end.
 // All state is FP64 structure-of-arrays; a step never synchronises the host.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -1864,6 +1864,18 @@ __global__ void k_ct_apply(DevRun r, const double* __restrict__ CT, double* __re
   for (int q = 0; q < 6; ++q) F[dir[q]][(size_t)var[q] * N + c] = CT[(size_t)q * N + c];
 }
 
+// The step's dt and next time from the reduced CFL bound (main.f90:763), by one
+// thread of the flux-CT pass: it runs after the reduction and before the
+// update, the first to read dt, in every stage, and writes the same values
+// each time.  (The last block of the reduction doing it cost 0.04 ms a step
+// on 256x128x128, its ticket being taken 32,000 times.)
+__device__ __forceinline__ void dt_body(const DevRun& r) {
+  Scal* s = r.scal;
+  const double dtcfl = __longlong_as_double((long long)s->dtcfl_bits);
+  s->dt = r.cfl * dtcfl;
+  s->timeh = s->time + s->dt;
+}
+
 // ---------------------------------------------------------------- flux-CT
 // ct.f90:30-118 (flux-CT, ict 1), ct.f90:121-233 (mflct, ict 2),
 // ct.f90:236-445 (upflct, ict 3: its last level) or none (ict 0) on nm1..n-nm1 in every dimension (edges with i in [ilo, ihi]),
@@ -1874,6 +1886,7 @@ __device__ __forceinline__ void ct_body(const DevRun& r, const S* __restrict__ F
                                             const S* __restrict__ F3, S* __restrict__ CT,
                                             float* __restrict__ CTcopy, int ilo, int ihi, const uint3 bid) {
   if (!r.scal->active) return;
+  if (bid.x == 0 && bid.y == 0 && bid.z == 0 && threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) dt_body(r);
   const int nm1 = r.nm1;
   const int i = bid.x * blockDim.x + threadIdx.x + ilo;
   const int j = jidx(r, nm1, bid);
@@ -2343,6 +2356,18 @@ __global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b, si
   if (x < n) b[x] = (float)a[x];
 }
 
+// ------------------------------------------------------ scalars of a step
+// The step's loop top (main.f90:617-620): its time, whether it is still
+// taken, and the start of the CFL reduction (cdtcfl.f90:30).  Run where the
+// step before it ends (k_step_end) and where a run's time is set (scal_begin
+// on the host does the same), so that a step opens with the reduction.
+__device__ __forceinline__ void step_begin_body(const DevRun& r) {
+  Scal* s = r.scal;
+  if (!s->active) return;
+  s->time = s->timeh;
+  if (s->time > r.tmax) { s->active = 0; return; }
+  s->dtcfl_bits = (unsigned long long)__double_as_longlong(1.0);
+}
 // ------------------------------------------------------------------- CFL
 // cdtcfl4 (cdtcfl.f90:2-129) with calcha4 (calcha.f90:129-367) over
 // is1+1..ie1-1 (every dimension); min over cells, then over blocks with an
@@ -2393,29 +2418,14 @@ __device__ __forceinline__ void cfl_body(const DevRun& r, const double* __restri
 }
 __global__ void __launch_bounds__(128, RG_CELL_MINB) k_cfl(DevRun r, const double* __restrict__ P) { cfl_body(r, P, blockIdx); }
 
-__device__ __forceinline__ void step_begin_body(const DevRun& r) {
-  Scal* s = r.scal;
-  if (!s->active) return;
-  s->time = s->timeh;  // main.f90:617-620
-  if (s->time > r.tmax) { s->active = 0; return; }
-  s->dtcfl_bits = (unsigned long long)__double_as_longlong(1.0);
-}
-__device__ __forceinline__ void dt_body(const DevRun& r) {
-  Scal* s = r.scal;
-  if (!s->active) return;
-  const double dtcfl = __longlong_as_double((long long)s->dtcfl_bits);
-  s->dt = r.cfl * dtcfl;  // main.f90:763
-  s->timeh = s->time + s->dt;
-}
 // The buffer rotation advances every step (a finished run copies its state
 // through the stages), the step count only while the run is active.
 __device__ __forceinline__ void step_end_body(const DevRun& r) {
   Scal* s = r.scal;
   s->cur = (s->cur + 1) % 3;
   if (s->active) atomicAdd(r.cnt + C_STEPS, 1ull);
+  step_begin_body(r);
 }
-__global__ void k_step_begin(DevRun r) { step_begin_body(r); }
-__global__ void k_dt(DevRun r) { dt_body(r); }
 __global__ void k_step_end(DevRun r) { step_end_body(r); }
 
 // ------------------------------------------------------ snapshot output
@@ -2802,14 +2812,6 @@ inline dim3 sgrid(const DevRun& r, int nx, int ny, int nz, dim3 b) {
 }  // namespace
 
 // ------------------------------------------------------------- launchers
-cudaError_t launch_step_begin(const DevRun& r, cudaStream_t s) {
-  k_step_begin<<<1, 1, 0, s>>>(r);
-  return cudaGetLastError();
-}
-cudaError_t launch_dt(const DevRun& r, cudaStream_t s) {
-  k_dt<<<1, 1, 0, s>>>(r);
-  return cudaGetLastError();
-}
 cudaError_t launch_step_end(const DevRun& r, cudaStream_t s) {
   k_step_end<<<1, 1, 0, s>>>(r);
   return cudaGetLastError();

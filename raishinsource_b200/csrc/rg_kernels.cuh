@@ -21,8 +21,6 @@ struct DevBufs {
 };
 
 cudaError_t launch_cfl(const DevRun& r, const double* P, cudaStream_t s);
-cudaError_t launch_step_begin(const DevRun& r, cudaStream_t s);
-cudaError_t launch_dt(const DevRun& r, cudaStream_t s);
 cudaError_t launch_step_end(const DevRun& r, cudaStream_t s);
 cudaError_t launch_flux(const DevRun& r, int dir, const double* P, double* F, cudaStream_t s);
 // Faces (PPM, MP5, WENO5, WENO-Z, WENO-M) of a run stored in full (no slab
