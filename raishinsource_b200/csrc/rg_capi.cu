@@ -13,6 +13,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/raishin_gpu.h"
@@ -344,12 +345,13 @@ Run* find(rg_ctx* ctx, int id) {
   return it == ctx->runs.end() ? nullptr : it->second;
 }
 
-int upload(const std::vector<double>& h, const double** dst, Run* R, cudaStream_t s) {
+template <typename T>
+int upload(const std::vector<T>& h, const T** dst, Run* R, cudaStream_t s) {
   void* p = nullptr;
-  int rc = dalloc(R, &p, h.size() * sizeof(double));
+  int rc = dalloc(R, &p, h.size() * sizeof(T));
   if (rc) return rc;
-  RG_CUDA(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-  *dst = static_cast<const double*>(p);
+  RG_CUDA(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+  *dst = static_cast<const T*>(p);
   return RG_OK;
 }
 
@@ -414,31 +416,35 @@ std::vector<double> shifted(const std::vector<double>& v, int n) {
 }
 
 // PPM's coefficients of one axis (PpmCoef in rg_recon.cuh) for the cells whose
-// stencil of spacings lies inside it, in FP64 as the reference writes them
+// stencil of spacings lies inside it, as the reference writes them
 // (rec.f90:1346-1468, 1479-1686); dx is rec2's shifted spacing, x the centres.
-std::vector<double> ppm_coefs(const Axis& ax, int n) {
+// T: the arithmetic of the faces that read them.
+template <typename T>
+std::vector<T> ppm_coefs(const Axis& ax, int n) {
   const std::vector<double> sh = shifted(ax.dxb, n);
-  auto dx = [&](int m) { return sh[m - 1]; };
-  std::vector<double> o(kPpmPlanes * (size_t)n, 0.0);
+  auto dx = [&](int m) { return T(sh[m - 1]); };
+  auto x = [&](int m) { return T(ax.x[m]); };
+  const T one = T(1), two = T(2);
+  std::vector<T> o(kPpmPlanes * (size_t)n, T(0));
   for (int m = 2; m <= n - 2; ++m) {
-    double* q = o.data() + m - 1;
-    const double a = dx(m - 1), b = dx(m), c = dx(m + 1), d = dx(m + 2);
+    T* q = o.data() + m - 1;
+    const T a = dx(m - 1), b = dx(m), c = dx(m + 1), d = dx(m + 2);
     q[0] = b / (a + b + c);
-    q[n] = (2.0 * a + b) / (c + b);
-    q[2 * n] = (b + 2.0 * c) / (a + b);
+    q[n] = (two * a + b) / (c + b);
+    q[2 * n] = (b + two * c) / (a + b);
     q[3 * n] = b / (b + c);
-    const double t3a = 1.0 / (a + b + c + d);
-    const double t3b = (2.0 * c * b) / (b + c);
-    const double t3c = ((a + b) / (2.0 * b + c)) - ((d + c) / (2.0 * c + b));
+    const T t3a = one / (a + b + c + d);
+    const T t3b = (two * c * b) / (b + c);
+    const T t3c = ((a + b) / (two * b + c)) - ((d + c) / (two * c + b));
     q[4 * n] = t3a * t3b * t3c;
-    q[5 * n] = t3a * b * ((a + b) / (2.0 * b + c));
-    q[6 * n] = t3a * c * ((c + d) / (b + 2.0 * c));
-    q[7 * n] = 1.0 / (a + b + c);
+    q[5 * n] = t3a * b * ((a + b) / (two * b + c));
+    q[6 * n] = t3a * c * ((c + d) / (b + two * c));
+    q[7 * n] = one / (a + b + c);
     q[8 * n] = c + b;
-    q[9 * n] = 1.0 / (c + b);
-    q[10 * n] = ax.x[m + 1] - ax.x[m - 1];
-    const double e = ax.x[m] - ax.x[m - 1], f = ax.x[m + 1] - ax.x[m];
-    q[11 * n] = e * e * e + f * f * f;
+    q[9 * n] = one / (c + b);
+    q[10 * n] = x(m + 1) - x(m - 1);
+    const T e = x(m) - x(m - 1), f = x(m + 1) - x(m);
+    q[11 * n] = std::is_same<T, float>::value ? std::fma(e * e, e, f * f * f) : e * e * e + f * f * f;
   }
   return o;
 }
@@ -1146,6 +1152,7 @@ int rg_run_admit_prep(rg_ctx* ctx, rg_prep* prep, int* run_id) {
   d.kmet = d.kfix;
   d.nik = (size_t)p->imax * (d.kfix ? 1 : p->kmax);
   d.gam1 = p->gam / (p->gam - 1.0);
+  d.gam1_32 = (float)p->gam / ((float)p->gam - 1.0f);
   d.gam = p->gam; d.cfl = p->cfl; d.dmin = p->dmin; d.pmin = p->pmin; d.pmax = p->pmax; d.tmax = p->tmax;
   std::memcpy(d.ibc, p->ibc, sizeof(d.ibc));
   d.carry_cap = kCarryCap;
@@ -1221,9 +1228,10 @@ int rg_run_admit_prep(rg_ctx* ctx, rg_prep* prep, int* run_id) {
   const int ext[3] = {p->imax, p->jmax, p->kmax};
   for (int a = 0; a < 3; ++a)
     if ((rc = upload(limiter_coefs(G.ax[a], ext[a], p->metric == 403, p->irec), &d.lim[a], R, s))) return bail(rc);
-  if (p->irec == 5)
-    for (int a = 0; a < 3; ++a)
-      if ((rc = upload(ppm_coefs(G.ax[a], ext[a]), &d.ppm[a], R, s))) return bail(rc);
+  for (int a = 0; a < 3 && p->irec == 5; ++a) {
+    if ((rc = upload(ppm_coefs<double>(G.ax[a], ext[a]), &d.ppm[a], R, s))) return bail(rc);
+    if (d.mixed && (rc = upload(ppm_coefs<float>(G.ax[a], ext[a]), &d.ppm32[a], R, s))) return bail(rc);
+  }
   // the caches and floor tables are this run's own allocations: fill their derived parts
   if (launch_geom_derive(d, const_cast<double*>(d.mc), const_cast<double*>(d.mi), const_cast<double*>(d.mk),
                          const_cast<double*>(d.fl_de), const_cast<double*>(d.fl_pr), s) != cudaSuccess)

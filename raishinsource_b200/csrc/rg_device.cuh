@@ -304,6 +304,30 @@ __device__ __forceinline__ void calucon(T u1, T u2, T u3, T gfl, const MetT<T>& 
   ucon[3] = u3;  // beta^theta = 0
 }
 
+// A product that is rounded by itself: the LLF flux subtracts the two states of
+// a face, and a product fused into that difference on one side only would
+// leave a rounding error where the states are equal.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+// Whether a face state spells out the roundings of products that enter two
+// sums.  Left to the compiler, one kernel fuses such a product into one of the
+// sums, another into none, and a face gets other last bits from the staged, the
+// direct and the batched kernel.  In FP64 that is 1e-16; in FP32 it can flip
+// MP5's switch (see gam1_of in rg_kernels.cu), so there every kernel rounds the
+// shared products by themselves and fuses the others.
+template <typename T>
+constexpr bool kPinned = sizeof(T) == 4;
+// A fused multiply-add in the product build, a product and a sum in the
+// uncontracted one.
+template <typename T>
+__device__ __forceinline__ T mad(T a, T b, T c) {
+#ifdef RG_EXACT_ARITH
+  return a * b + c;
+#else
+  return fma(a, b, c);
+#endif
+}
+
 // Velocity and magnetic 4-vectors of one primitive state (the common head of
 // caluu1/caluu3/calflx3*/caltenr, caluu.f90:40-90).
 template <typename T>
@@ -316,7 +340,9 @@ using PS = PST<double>;
 
 // The state of q with a given Lorentz factor gfl (pstate below computes it
 // with calgfl; the output converter uses its own clamps).  gam1 = gam/(gam-1).
-template <typename T, typename M>
+// D: the direction of the face the state belongs to (its flux and conserved
+// energy share b^D b_D and b^t b_t with b^2), 0 for a state at a cell.
+template <int D = 0, typename T, typename M>
 __device__ __forceinline__ void pstate_gfl(const T q[9], const MetT<T>& m, T gam1, T gfl, PST<T>& s, M& ma) {
   s.de = q[0];
   s.pr = q[4];
@@ -332,11 +358,18 @@ __device__ __forceinline__ void pstate_gfl(const T q[9], const MetT<T>& m, T gam
   s.bbcon[2] = (s.b2 + s.bbcon[0] * s.ucon[2]) * s.iu0;
   s.bbcon[3] = (s.b3 + s.bbcon[0] * s.ucon[3]) * s.iu0;
   lower_g(s.bbcon, s.bbcov, m);
-  s.bbsq = s.bbcon[0] * s.bbcov[0] + s.bbcon[1] * s.bbcov[1] + s.bbcon[2] * s.bbcov[2] + s.bbcon[3] * s.bbcov[3];
+  if constexpr (D > 0 && kPinned<T>) {
+    s.bbsq = mul_rn(s.bbcon[0], s.bbcov[0]);
+#pragma unroll
+    for (int n = 1; n <= 3; ++n)
+      s.bbsq = n == D ? s.bbsq + mul_rn(s.bbcon[n], s.bbcov[n]) : fma(s.bbcon[n], s.bbcov[n], s.bbsq);
+  } else {
+    s.bbsq = s.bbcon[0] * s.bbcov[0] + s.bbcon[1] * s.bbcov[1] + s.bbcon[2] * s.bbcov[2] + s.bbcon[3] * s.bbcov[3];
+  }
 }
-template <typename T, typename M>
+template <int D = 0, typename T, typename M>
 __device__ __forceinline__ void pstate(const T q[9], const MetT<T>& m, T gam1, PST<T>& s, M& ma) {
-  pstate_gfl(q, m, gam1, calgfl(q[1], q[2], q[3], m, ma), s, ma);
+  pstate_gfl<D>(q, m, gam1, calgfl(q[1], q[2], q[3], m, ma), s, ma);
 }
 template <typename T>
 __device__ __forceinline__ void pstate(const T q[9], const MetT<T>& m, T gam1, PST<T>& s) {
@@ -355,21 +388,17 @@ __device__ __forceinline__ T ent_ratio(const PST<T>& s, T gam, int gkind) {
   return ent_ratio(s, gam, gkind, ma);
 }
 
-// A product that is rounded by itself: the LLF flux subtracts the two states of
-// a face, and a product fused into that difference on one side only would
-// leave a rounding error where the states are equal.
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-
 // caluu.f90:92-118: sqrt(-g) (rho u^t, T^t_i, T^t_t + rho u^t, s u^t, B^i).
 // delta(0,n) is the literal identity of caldelta (physfunc.f90:122-158).
 template <typename T, bool FACE = false>
 __device__ __forceinline__ void p2c(const PST<T>& s, T gam, T detg, T u[9], T sr) {
   const T a = s.roh + s.bbsq, b = s.pr + T(0.5) * s.bbsq;
-  u[0] = s.de * s.ucon[0];
+  constexpr bool pin = FACE && kPinned<T>;
+  u[0] = pin ? mul_rn(s.de, s.ucon[0]) : s.de * s.ucon[0];
 #pragma unroll
   for (int m = 1; m <= 3; ++m) u[m] = a * s.ucon[0] * s.ucov[m] + b * T(0) - s.bbcon[0] * s.bbcov[m];
-  u[4] = a * s.ucon[0] * s.ucov[0] + b * T(1) - s.bbcon[0] * s.bbcov[0] + s.de * s.ucon[0];
+  if (pin) u[4] = fma(a * s.ucon[0], s.ucov[0], b) - mul_rn(s.bbcon[0], s.bbcov[0]) + u[0];
+  else u[4] = a * s.ucon[0] * s.ucov[0] + b * T(1) - s.bbcon[0] * s.bbcov[0] + s.de * s.ucon[0];
   u[5] = s.de * sr * s.ucon[0];
   u[6] = s.b1; u[7] = s.b2; u[8] = s.b3;
 #pragma unroll
@@ -387,10 +416,13 @@ __device__ __forceinline__ void flux(const PST<T>& s, T gam, T detg, T w[9], T s
   const T a = s.roh + s.bbsq, b = s.pr + T(0.5) * s.bbsq;
   const T ud = s.ucon[D];
   const T bc[4] = {T(0), s.b1, s.b2, s.b3};
-  w[0] = s.de * ud;
+  w[0] = kPinned<T> ? mul_rn(s.de, ud) : s.de * ud;
 #pragma unroll
-  for (int m = 1; m <= 3; ++m) w[m] = a * ud * s.ucov[m] + b * (D == m ? T(1) : T(0)) - s.bbcon[D] * s.bbcov[m];
-  w[4] = a * ud * s.ucov[0] + b * T(0) - s.bbcon[D] * s.bbcov[0] + s.de * ud;
+  for (int m = 1; m <= 3; ++m) {
+    if (m == D && kPinned<T>) w[m] = fma(a * ud, s.ucov[m], b) - mul_rn(s.bbcon[m], s.bbcov[m]);
+    else w[m] = a * ud * s.ucov[m] + b * (D == m ? T(1) : T(0)) - s.bbcon[D] * s.bbcov[m];
+  }
+  w[4] = a * ud * s.ucov[0] + b * T(0) - s.bbcon[D] * s.bbcov[0] + (kPinned<T> ? w[0] : s.de * ud);
   w[5] = s.de * sr * ud;
 #pragma unroll
   for (int m = 1; m <= 3; ++m) {

@@ -1021,6 +1021,22 @@ template <>
 __device__ __forceinline__ const float* met_of<2, float>(const DevRun& r) { return r.mc32; }
 template <>
 __device__ __forceinline__ const float* met_of<3, float>(const DevRun& r) { return r.mk32; }
+// Constants that depend on the arithmetic type, each evaluated in it: a last bit
+// of an FP32 constant moves every FP32 face, and MP5's switch between its
+// unlimited and limited value (an absolute 1e-10, far below FP32's resolution)
+// turns a last bit into a jump.
+template <typename T>
+__device__ __forceinline__ T gam1_of(const DevRun& r);
+template <>
+__device__ __forceinline__ double gam1_of<double>(const DevRun& r) { return r.gam1; }
+template <>
+__device__ __forceinline__ float gam1_of<float>(const DevRun& r) { return r.gam1_32; }
+template <typename T>
+__device__ __forceinline__ const T* ppm_of(const DevRun& r, int axis);
+template <>
+__device__ __forceinline__ const double* ppm_of<double>(const DevRun& r, int axis) { return r.ppm[axis]; }
+template <>
+__device__ __forceinline__ const float* ppm_of<float>(const DevRun& r, int axis) { return r.ppm32[axis]; }
 
 //
 // OUT (the per-routine rg_rec2): the lane also stores its face state, face
@@ -1054,7 +1070,7 @@ __device__ __forceinline__ void face_recon(const DevRun& r, const S* __restrict_
   if (IREC == 5) {
     const int f = ((D == 1) ? i : (D == 2 ? j : k)) + side;  // owner cell of this lane's state
     const int n = (D == 1) ? r.imax : (D == 2 ? r.jmax : r.kmax);
-    ppm_cell<D, T, S, OUT>(Pv + cv + side * sv, Nv, sv, r.ppm[D - 1] + f - 1, n, T(r.gam), side, q);
+    ppm_cell<D, T, S, OUT>(Pv + cv + side * sv, Nv, sv, ppm_of<T>(r, D - 1) + f - 1, n, T(r.gam), side, q);
   } else if (IREC == 1 || IREC == 2 || IREC == 11 || IREC == 12 || IREC == 13) {
     // owner cell f of this lane's state and its coordinate's coefficients
     const int f = ((D == 1) ? i : (D == 2 ? j : k)) + side;
@@ -1160,7 +1176,7 @@ template <int D, typename T, typename M>
 __device__ __forceinline__ void face_state_m(const T q[9], const MetT<T>& m, T gam, T gam1, int gkind, FaceSt<T>& o,
                                              M& ma) {
   PST<T> s;
-  pstate(q, m, gam1, s, ma);
+  pstate<D>(q, m, gam1, s, ma);
   const T sr = ent_ratio(s, gam, gkind, ma);
   p2c<T, true>(s, gam, m.detg, o.u, sr);
   flux<D>(s, gam, m.detg, o.w, sr);
@@ -1213,7 +1229,7 @@ __device__ __forceinline__ void face_lane(const DevRun& r, const S* __restrict__
   MetT<T> m;
   load_met(met_of<D, S>(r), r.nik, r.ik(i, k), m);
   FaceSt<T> s;
-  face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, s);
+  face_state<D, T>(q, m, T(r.gam), gam1_of<T>(r), r.gkind, s);
   if constexpr (OUT) {
     if (valid) {
 #pragma unroll
@@ -1267,7 +1283,7 @@ __device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, 
   FaceSt<T> L, R;
   if constexpr (IREC == 5) {
     const int f = (D == 1) ? i : (D == 2 ? j : k), n = (D == 1) ? r.imax : (D == 2 ? r.jmax : r.kmax);
-    const double* pc = r.ppm[D - 1] + f - 1;
+    const T* pc = ppm_of<T>(r, D - 1) + f - 1;
     q[5] = qR[5] = T(0);
     if constexpr (STASH) {
       // through the slots: the left state in 0-8, the right one in 9-17, which
@@ -1290,7 +1306,7 @@ __device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, 
   } else {
     face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 0, q);
   }
-  face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, L);
+  face_state<D, T>(q, m, T(r.gam), gam1_of<T>(r), r.gkind, L);
   if (IREC == 5) {
     if (STASH)
 #pragma unroll
@@ -1314,7 +1330,7 @@ __device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, 
   } else {
     face_recon<D, IREC, T, S, false, true>(r, nullptr, Vp, Vn, Vc, Vst, i, j, k, 1, q);
   }
-  face_state<D, T>(q, m, T(r.gam), T(r.gam1), r.gkind, R);
+  face_state<D, T>(q, m, T(r.gam), gam1_of<T>(r), r.gkind, R);
   T cmax, c1;
   face_bounds<D, T>(vpL, vmL, R.vp, R.vm, cmax, c1);
   const size_t N = r.N, c = r.cell(i, j, k);

@@ -94,31 +94,37 @@ __device__ __forceinline__ T mp5_value(T a2, T a1, T u0, T b1, T b2) {
 
 // The convex combination of the three candidates with the weights n_m / d_m
 // as the reference forms it: six quotients.
-#ifdef RG_EXACT_ARITH
-#define RG_WENO_QUOT __forceinline__
-#else
-#define RG_WENO_QUOT __noinline__
-#endif
 template <typename T>
-__device__ RG_WENO_QUOT T weno_quot(T n0, T d0, T n1, T d1, T n2, T d2, T q0, T q1, T q2) {
+__device__ __forceinline__ T weno_quot(T n0, T d0, T n1, T d1, T n2, T d2, T q0, T q1, T q2) {
   const T w0 = n0 / d0, w1 = n1 / d1, w2 = n2 / d2;
   const T wt = w0 + w1 + w2;
   const T o0 = w0 / wt, o1 = w1 / wt, o2 = w2 / wt;
   return o0 * q0 + o1 * q1 + o2 * q2;
 }
-// The same with weights already multiplied by their common denominator, which
-// leaves one reciprocal.  Where the products leave the range in which they
-// and the reciprocal are exact to rounding (fields beyond about 1e37 in FP64 or
-// 1e4 in FP32, non-finite values), `quot` forms the quotients instead.
-template <typename T, typename F>
-__device__ __forceinline__ T weno_mean(T w0, T w1, T w2, T q0, T q1, T q2, const F& quot) {
-  const T wt = w0 + w1 + w2;
-  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p120f), small = sizeof(T) == 8 ? T(0x1p-500) : T(0x1p-100f);
-  if (!(wt < big && wt > small)) return quot();
-  const T o = w0 * q0 + w1 * q1 + w2 * q2;
-  if constexpr (sizeof(T) == 8) return o * rcp_newton(wt);
-  else return mdiv(o, wt);
+// Out of line, for FP64 states that hardly ever take it.
+__device__ __noinline__ double weno_quot_rare(double n0, double d0, double n1, double d1, double n2, double d2,
+                                              double q0, double q1, double q2) {
+  return weno_quot(n0, d0, n1, d1, n2, d2, q0, q1, q2);
 }
+// The same in FP64 with weights already multiplied by their common denominator,
+// which leaves one reciprocal.  Where the products leave the range in which
+// they and the reciprocal are exact to rounding (fields beyond about 1e37,
+// non-finite values), `quot` forms the quotients instead.  FP32 states always
+// form them: the products of six small weights keep too little of FP32's range.
+template <typename F>
+__device__ __forceinline__ double weno_mean(double w0, double w1, double w2, double q0, double q1, double q2,
+                                            const F& quot) {
+  const double wt = w0 + w1 + w2;
+  if (!(wt < 0x1p500 && wt > 0x1p-500)) return quot();
+  return (w0 * q0 + w1 * q1 + w2 * q2) * rcp_newton(wt);
+}
+#ifdef RG_EXACT_ARITH
+template <typename T>
+constexpr bool kWenoMean = false;
+#else
+template <typename T>
+constexpr bool kWenoMean = sizeof(T) == 8;
+#endif
 
 // rec.f90:2373-2643 (WENO5-JS); the left state at +1/2 takes
 // (u-2, u-1, u0, u+1, u+2), the right state at -1/2 the mirrored stencil.
@@ -141,17 +147,15 @@ __device__ __forceinline__ T weno5_js(T a2, T a1, T u0, T b1, T b2, T b1s) {
   const T q0 = c00 * a2 + c01 * a1 + c02 * u0;
   const T q1 = c10 * a1 + c11 * u0 + c12 * b1;
   const T q2 = c20 * u0 + c21 * b1 + c22 * b2;
-#ifndef RG_EXACT_ARITH
-  {
+  if constexpr (kWenoMean<T>) {
     // the weights cd_m / beta_m^2 times (beta_0 beta_1 beta_2)^2
     const T p0 = be1 * be2, p1 = be0 * be2, p2 = be0 * be1;
     return weno_mean(cd0 * (p0 * p0), cd1 * (p1 * p1), cd2 * (p2 * p2), q0, q1, q2, [&] {
-      return weno_quot(cd0, be0 * be0, cd1, be1 * be1, cd2, be2 * be2, q0, q1, q2);
+      return weno_quot_rare(cd0, be0 * be0, cd1, be1 * be1, cd2, be2 * be2, q0, q1, q2);
     });
+  } else {
+    return weno_quot(cd0, be0 * be0, cd1, be1 * be1, cd2, be2 * be2, q0, q1, q2);
   }
-#else
-  return weno_quot(cd0, be0 * be0, cd1, be1 * be1, cd2, be2 * be2, q0, q1, q2);
-#endif
 }
 template <typename T>
 __device__ __forceinline__ T weno5_state(T a2, T a1, T u0, T b1, T b2) {
@@ -186,14 +190,14 @@ __device__ __forceinline__ T weno5z_state(T a2, T a1, T u0, T b1, T b2) {
     const T o0 = w0 / wt, o1 = w1 / wt, o2 = w2 / wt;
     return o0 * q0 + o1 * q1 + o2 * q2;
   };
-#ifndef RG_EXACT_ARITH
-  // the weights times the product of the beta_m + eps
-  const T e0 = be0 + epsi, e1 = be1 + epsi, e2 = be2 + epsi;
-  return weno_mean(cd0 * (e0 + tau) * (e1 * e2), cd1 * (e1 + tau) * (e0 * e2), cd2 * (e2 + tau) * (e0 * e1), q0, q1,
-                   q2, quot);
-#else
-  return quot();
-#endif
+  if constexpr (kWenoMean<T>) {
+    // the weights times the product of the beta_m + eps
+    const T e0 = be0 + epsi, e1 = be1 + epsi, e2 = be2 + epsi;
+    return weno_mean(cd0 * (e0 + tau) * (e1 * e2), cd1 * (e1 + tau) * (e0 * e2), cd2 * (e2 + tau) * (e0 * e1), q0, q1,
+                     q2, quot);
+  } else {
+    return quot();
+  }
 }
 
 // rec.f90:3439-3793 (mapped WENO5, Henrick et al. 2005): the JS weights
@@ -229,8 +233,7 @@ __device__ __forceinline__ T weno5m_state(T a2, T a1, T u0, T b1, T b2) {
     const T o0 = g[0] / gt, o1 = g[1] / gt, o2 = g[2] / gt;
     return o0 * q0 + o1 * q1 + o2 * q2;
   };
-#ifndef RG_EXACT_ARITH
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (kWenoMean<T>) {
     // the weights times (beta_0 + eps)^2 (beta_1 + eps)^2 (beta_2 + eps)^2, the
     // beta_m + eps (at least 1e-40) scaled by 2^60 to keep the products from
     // underflowing; the mapped weights over their common denominator
@@ -250,9 +253,9 @@ __device__ __forceinline__ T weno5m_state(T a2, T a1, T u0, T b1, T b2) {
     }
     return weno_mean(num[0] * (den[1] * den[2]), num[1] * (den[0] * den[2]), num[2] * (den[0] * den[1]), q0, q1, q2,
                      quot);
+  } else {
+    return quot();
   }
-#endif
-  return quot();
 }
 
 // The second-order limiters of rec.f90 on nonuniform coordinates: mclim
@@ -362,7 +365,8 @@ __device__ __forceinline__ T muscl_state(T um, T u0, T up, int side) {
 // The coefficients of the spacings are the run's (PpmCoef planes of
 // DevRun::ppm, rg_capi.cu): each is the reference's expression in its order,
 // evaluated once per index instead of once per cell, variable and face (about
-// 40 divisions a cell and variable), so the values are the same.
+// 40 divisions a cell and variable), so the values are the same.  FP32 faces
+// have planes of their own, evaluated in FP32 from the rounded spacings.
 // Planes at 0-based index m-1, with dx(m) the shifted spacing:
 enum PpmCoef {
   PC_A = 0,  // dx(m) / (dx(m-1) + dx(m) + dx(m+1))
@@ -407,7 +411,7 @@ __device__ __forceinline__ double ppm_over(double a, double b, double rb) {
   return div_by_rcp(a, b, rb);
 #endif
 }
-__device__ __forceinline__ float ppm_over(float a, float, float rb) { return a * rb; }
+__device__ __forceinline__ float ppm_over(float a, float b, float) { return a / b; }
 
 // The contact steepening factor (detect, rec.f90:1479-1686) and the shock
 // flattening factor f2a (flaten, rec.f90:1689-1884) of the cell `o` cells above
@@ -466,11 +470,18 @@ __device__ __forceinline__ void ppm_factors(const FU& U, const FC& C, int o, T g
   }
 }
 
+// r (1 - w) + x w, its roundings spelled out: it sums two products, and a face
+// gets the same bits whichever kernel forms it.
+template <typename T>
+__device__ __forceinline__ T ppm_blend(T r, T x, T w) {
+  return mad(x, w, mul_rn(r, T(1.0) - w));
+}
+
 // flaten's blend and monoto (rec.f90:1887-2056) of one cell's states.
 template <typename T>
 __device__ __forceinline__ void ppm_monoto(T u0, T f2a, T& l, T& r) {
-  r = u0 * f2a + r * (T(1.0) - f2a);
-  l = u0 * f2a + l * (T(1.0) - f2a);
+  r = ppm_blend(r, u0, f2a);
+  l = ppm_blend(l, u0, f2a);
   if ((r - u0) * (l - u0) >= T(0)) { r = u0; l = u0; }
   const T t3 = T(6.0) * (r - l) * (u0 - T(0.5) * (r + l));
   const T t4 = (r - l) * (r - l);
@@ -484,10 +495,10 @@ __device__ __forceinline__ void ppm_monoto(T u0, T f2a, T& l, T& r) {
 // test (rec.f90:1623).  ALL: also the sixth variable (the per-routine rec2
 // outputs every face state).
 template <int D, typename T, typename S, bool ALL>
-__device__ __forceinline__ void ppm_cell(const S* __restrict__ p, size_t N, long long st, const double* __restrict__ pc,
+__device__ __forceinline__ void ppm_cell(const S* __restrict__ p, size_t N, long long st, const T* __restrict__ pc,
                                          int n, T gam, int side, T q[9]) {
   auto U = [&](int v, int o) { return T(p[(size_t)v * N + o * st]); };
-  auto C = [&](int a, int o) { return T(__ldg(pc + a * n + o)); };
+  auto C = [&](int a, int o) { return __ldg(pc + a * n + o); };
   T eta, f2a;
   ppm_factors<D, T>(U, C, 0, gam, eta, f2a);
 #pragma unroll 1
@@ -501,8 +512,8 @@ __device__ __forceinline__ void ppm_cell(const S* __restrict__ p, size_t N, long
       T l = ppm_face(um1, u0, dm, d0, C(PC_T2, -1), C(PC_T3, -1), C(PC_T4, -1), C(PC_T5, -1));
       T r = ppm_face(u0, up1, d0, dp, C(PC_T2, 0), C(PC_T3, 0), C(PC_T4, 0), C(PC_T5, 0));
       if (v == 0) {
-        r = r * (T(1.0) - eta) + (up1 - T(0.5) * dp) * eta;
-        l = l * (T(1.0) - eta) + (um1 + T(0.5) * dm) * eta;
+        r = ppm_blend(r, up1 - T(0.5) * dp, eta);
+        l = ppm_blend(l, um1 + T(0.5) * dm, eta);
       }
       ppm_monoto(u0, f2a, l, r);
       o = side ? l : r;
@@ -521,9 +532,9 @@ __device__ __forceinline__ void ppm_cell(const S* __restrict__ p, size_t N, long
 // then leave room in the registers; put must take a run-time v).
 template <int D, typename T, typename S, bool PACK, bool ROLL, typename Put>
 __device__ __forceinline__ void ppm_face_pair(const S* __restrict__ p, size_t N, long long st,
-                                              const double* __restrict__ pc, int n, T gam, const Put& put) {
+                                              const T* __restrict__ pc, int n, T gam, const Put& put) {
   auto U = [&](int v, int o) { return T(p[(size_t)(PACK && v > 5 ? v - 1 : v) * N + o * st]); };
-  auto C = [&](int a, int o) { return T(__ldg(pc + a * n + o)); };
+  auto C = [&](int a, int o) { return __ldg(pc + a * n + o); };
   T etaL, fL, etaR, fR;
   ppm_factors<D, T>(U, C, 0, gam, etaL, fL);
   ppm_factors<D, T>(U, C, 1, gam, etaR, fR);
@@ -542,10 +553,10 @@ __device__ __forceinline__ void ppm_face_pair(const S* __restrict__ p, size_t N,
     for (int o = 0; o < 3; ++o) f[o] = ppm_face(u[o + 1], u[o + 2], d[o], d[o + 1], t2[o], t3[o], t4[o], t5[o]);
     T l0 = f[0], r0 = f[1], l1 = f[1], r1 = f[2];
     if (v == 0) {
-      r0 = r0 * (T(1.0) - etaL) + (u[3] - T(0.5) * d[2]) * etaL;
-      l0 = l0 * (T(1.0) - etaL) + (u[1] + T(0.5) * d[0]) * etaL;
-      r1 = r1 * (T(1.0) - etaR) + (u[4] - T(0.5) * d[3]) * etaR;
-      l1 = l1 * (T(1.0) - etaR) + (u[2] + T(0.5) * d[1]) * etaR;
+      r0 = ppm_blend(r0, u[3] - T(0.5) * d[2], etaL);
+      l0 = ppm_blend(l0, u[1] + T(0.5) * d[0], etaL);
+      r1 = ppm_blend(r1, u[4] - T(0.5) * d[3], etaR);
+      l1 = ppm_blend(l1, u[2] + T(0.5) * d[1], etaR);
     }
     ppm_monoto(u[2], fL, l0, r0);
     ppm_monoto(u[3], fR, l1, r1);

@@ -75,6 +75,7 @@ struct DevRun {
   size_t nik;            // (i,k) points of the metric caches (imax for a theta slab)
   double gam, cfl, dmin, pmin, pmax, tmax;
   double gam1;           // gam/(gam-1)
+  float gam1_32;         // the same evaluated in FP32, as the FP32 faces' other constants are
   const double* mc;      // metric at cell centres (also the phi faces)
   const double* mi;      // metric at the r faces x1a(i)
   const double* mk;      // metric at the theta faces x3a(k)
@@ -97,6 +98,7 @@ struct DevRun {
   // PPM's coefficients of the spacings per direction (PpmCoef in rg_recon.cuh,
   // kPpmCoef planes of n_d values at index m-1; only for irec 5)
   const double* ppm[3];
+  const float* ppm32[3];  // the same evaluated in FP32 (mixed runs)
   // Limiter coefficients per direction d (MC, minmod, LimO3, MVL, Koren,
   // CENO): ten planes of n_d values at index m-1 of the cell's coordinate
   // spacings, as limiter_state and ceno_state in rg_recon.cuh read them.
