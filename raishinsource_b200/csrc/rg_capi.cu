@@ -116,6 +116,7 @@ struct rg_ctx {
   cudaEvent_t marks[RG_MAX_MARKS] = {};  // rg_ctx_mark / rg_ctx_wait_mark
   cudaStream_t side[2] = {nullptr, nullptr};  // the phi and theta faces of small 3D runs (run_stage)
   cudaEvent_t fork[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t read_done = nullptr;     // the caller's array of an upload has been read (to_soa)
   // pinned host memory that kernels write: one word (uploaded data not uniform), and from byte 64 the counters of
   // rg_calflx_static, whose call must read them without a device copy
   int* flag = nullptr;
@@ -555,19 +556,23 @@ int ensure_aos(Run* R) {
 }
 
 // Host reference-layout array -> device SoA in the layout of view v (the run's
-// stored layout, or the full layout of the per-routine entry points).  With
-// check, data that are not uniform along a slab direction are refused.
-int to_soa(rg_ctx* ctx, Run* R, const double* host_aos, double* dev_soa, const DevRun& v, bool check) {
+// stored layout, or the full layout of the per-routine entry points).  An
+// upload (the whole call: no result comes back behind which the caller waits)
+// refuses data that are not uniform along a slab direction and returns when
+// the caller's array has been read; what follows the read may still be queued.
+int to_soa(rg_ctx* ctx, Run* R, const double* host_aos, double* dev_soa, const DevRun& v, bool is_upload) {
   // an array on this device is read where it is; any other is copied to the
   // run's staging buffer first (cudaMemcpyDefault: host memory or another device's)
   const double* src = host_aos;
-  if (!device_array(ctx, host_aos)) {
+  const bool in_place = device_array(ctx, host_aos);
+  if (!in_place) {
     const int rc = ensure_aos(R);
     if (rc) return rc;
     RG_CUDA(cudaMemcpyAsync(R->aos, host_aos, 9 * R->nfull * sizeof(double), cudaMemcpyDefault, ctx->stream));
+    if (is_upload) RG_CUDA(cudaEventRecord(ctx->read_done, ctx->stream));
     src = R->aos;
   }
-  const bool verify = check && (v.jfix || v.kfix);
+  const bool verify = is_upload && (v.jfix || v.kfix);
   if (verify) *ctx->flag = 0;
   RG_CUDA(launch_aos_to_soa(v, src, dev_soa, verify ? ctx->flag : nullptr, ctx->stream));
   if (verify) {
@@ -576,6 +581,9 @@ int to_soa(rg_ctx* ctx, Run* R, const double* host_aos, double* dev_soa, const D
       return fail(RG_EINVAL_CONFIG,
                   "primitives differ along a slab direction (the run stores one plane of it); admit the run "
                   "with flags bit 0 (RG_FLAG_FULL) to compute every cell");
+  } else if (is_upload) {
+    if (in_place) RG_CUDA(cudaEventRecord(ctx->read_done, ctx->stream));
+    RG_CUDA(cudaEventSynchronize(ctx->read_done));
   }
   return RG_OK;
 }
@@ -984,8 +992,8 @@ int rg_ctx_create(int device, rg_ctx** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   for (cudaStream_t& t : c->side)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking);
-  for (cudaEvent_t& t : c->fork)
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t, cudaEventDisableTiming);
+  for (cudaEvent_t* t : {&c->fork[0], &c->fork[1], &c->fork[2], &c->read_done})
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(t, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     cudaFreeHost(c->flag);
     delete c;
@@ -1008,6 +1016,7 @@ int rg_ctx_destroy(rg_ctx* ctx) {
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   for (cudaStream_t t : ctx->side) cudaStreamDestroy(t);
   for (cudaEvent_t t : ctx->fork) cudaEventDestroy(t);
+  cudaEventDestroy(ctx->read_done);
   cudaFreeHost(ctx->flag);
   delete ctx;
   return RG_OK;

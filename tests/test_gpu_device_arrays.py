@@ -34,6 +34,23 @@ def test_device_upload_and_download_equal_host(gpu_ctx, kw, offset):
     r.release()
 
 
+@pytest.mark.parametrize("where", ["pinned", "device"])
+def test_upload_has_read_the_array_when_it_returns(gpu_ctx, where):
+    """A 3D run (no uniformity check to wait for), with steps queued ahead of
+    the upload: the array is overwritten as soon as the call returns."""
+    import torch
+    r = gpu_ctx.admit(dict(config.torus(nr=96, nth=64, nph=48), guard=1))
+    r.ic_torus(seed=9)
+    u = torch.from_numpy(r.prims())
+    buf = u.clone().pin_memory() if where == "pinned" else u.cuda()
+    torch.cuda.synchronize()
+    r.step(20)
+    r.upload_prims_ptr(buf.data_ptr(), t0=0.0)
+    buf.fill_(-7.0)
+    assert np.array_equal(r.prims(), u.numpy())
+    r.release()
+
+
 def test_device_upload_refuses_a_slab_that_is_not_uniform(gpu_ctx):
     import torch
     r = gpu_ctx.admit(dict(config.torus(nr=48, nth=40), guard=1))
