@@ -43,29 +43,34 @@ __device__ __forceinline__ float mdiv(float a, float b) { return __fdividef(a, b
 template <typename T>
 __device__ __forceinline__ T mrcp(T x) { return mdiv(T(1), x); }
 
-
 // Division, reciprocal and square root as the state functions below call
 // them, one instance per state.  IeeeMath: the operators above.  NewtonMath
-// (FP64): without the branches of a full IEEE operator, so that the
-// independent quotients of a state overlap instead of standing one behind
-// the other.  A reciprocal starts from the hardware's approximation
-// (rcp.approx.ftz.f64, about 20 bits), takes one third-order step of the
-// geometric series of 1/(1 - e), e = 1 - x y, and one Newton step on the
-// residual; a quotient corrects a y by its residual; a square root runs
-// the coupled (Goldschmidt) iteration from rsqrt.approx.ftz.f64 and corrects
-// by its residual (P. Markstein, IBM J. Res. Dev. 34, 1990; "Software
-// division and square root using Goldschmidt's algorithms", 2004).  With
-// operands whose magnitudes lie in [2^-500, 2^500) no step over- or underflows
-// and the results are the correctly rounded ones, save the reciprocal of a
-// significand of all ones, whose last bit is one too low: 1 - 2^-53, the value
-// below one that 1 - x takes for tiny x, is put right by rcp1().  note() collects the
-// operands' exponents and ok() tells whether all of them lay there.  A caller
-// that finds ok() false repeats the computation with IeeeMath (zeros,
-// subnormal, huge or non-finite operands).
+// (FP64, product build): without the branches of a full IEEE operator, so that
+// the independent quotients of a state overlap instead of standing one behind
+// the other; its operations are Goldschmidt's iterations as P. Markstein gives
+// them ("Software division and square root using Goldschmidt's algorithms",
+// 2004), closed by the residual corrections of his "Computation of elementary
+// functions on the IBM RISC System/6000 processor" (IBM J. Res. Dev. 34, 1990):
+//   reciprocal   y of the hardware's approximation (rcp.approx.ftz.f64, about
+//                20 bits), e = 1 - x y; y (1 + e)(1 + e^2) = y / (1 - e) to
+//                e^4; then y + y (1 - x y), which from a y within an ulp rounds
+//                1/x correctly unless x's significand is all ones
+//   quotient     q = a y, then q + y (a - b q): correctly rounded for a
+//                correctly rounded reciprocal y
+//   square root  g, h towards sqrt(x), 1/(2 sqrt(x)) from rsqrt.approx.ftz.f64
+//                by g + g e, h + h e with e = 1/2 - g h, twice, then
+//                g + h (x - g^2)
+// With operands whose magnitudes lie in [2^-500, 2^500) no step over- or
+// underflows.  note() collects the operands' exponents, divisor() also sees a
+// significand of all ones (1 - x gives one for tiny x; the low word alone is
+// looked at, one compare), and ok() tells whether every operand was in order.
+// A caller that finds ok() false repeats the computation with IeeeMath (zeros,
+// subnormal, huge or non-finite operands, the divisors above), so the values
+// are IEEE's in every case.  MP5 step of 256x128x128: 5.14 ms (5.16 with three
+// plain Newton steps in the reciprocal).
 template <typename T>
 struct IeeeMath {
   __device__ __forceinline__ T rcp(T x) { return mrcp(x); }
-  __device__ __forceinline__ T rcp1(T x) { return mrcp(x); }  // of a difference from one
   __device__ __forceinline__ T div(T a, T b) { return mdiv(a, b); }
   __device__ __forceinline__ T sqrt(T x) { return msqrt(x); }
   __device__ __forceinline__ bool ok() const { return true; }
@@ -73,11 +78,10 @@ struct IeeeMath {
 __device__ __forceinline__ double rcp_newton(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  e = fma(e, e, e);
+  const double e = fma(-x, y, 1.0);
   y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
+  y = fma(y, e * e, y);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 // a / b given y = 1/b correctly rounded
 __device__ __forceinline__ double div_by_rcp(double a, double b, double y) {
@@ -98,24 +102,35 @@ __device__ __forceinline__ double sqrt_newton(double x) {
 }
 struct NewtonMath {
   unsigned lo = 0x7fffffffu, hi = 0u;
+  bool ones = false;
   __device__ __forceinline__ void note(double x) {
     const unsigned a = (unsigned)__double2hiint(x) & 0x7fffffffu;
     lo = min(lo, a);
     hi = max(hi, a);
   }
-  __device__ __forceinline__ double rcp(double x) { note(x); return rcp_newton(x); }
-  __device__ __forceinline__ double rcp1(double x) {
-    const double y = rcp(x);
-    return x == 0x1.fffffffffffffp-1 ? 0x1.0000000000001p0 : y;
+  __device__ __forceinline__ void divisor(double x) {
+    note(x);
+    ones |= __double2loint(x) == -1;
   }
-  __device__ __forceinline__ double div(double a, double b) { note(a); note(b); return div_by_rcp(a, b, rcp_newton(b)); }
+  __device__ __forceinline__ double rcp(double x) { divisor(x); return rcp_newton(x); }
+  __device__ __forceinline__ double div(double a, double b) {
+    note(a);
+    divisor(b);
+    return div_by_rcp(a, b, rcp_newton(b));
+  }
   __device__ __forceinline__ double sqrt(double x) { note(x); return sqrt_newton(x); }
-  __device__ __forceinline__ bool ok() const { return lo >= (1023u - 500u) << 20 && hi < (1023u + 500u) << 20; }
+  __device__ __forceinline__ bool ok() const {
+    return lo >= (1023u - 500u) << 20 && hi < (1023u + 500u) << 20 && !ones;
+  }
 };
+// The operators of the face states: FP32 has its approximate ones already, the
+// uncontracted build takes IEEE's alone.
 template <typename T>
-struct FastMath : IeeeMath<T> {};  // FP32: the approximate operators already
+struct FastMath : IeeeMath<T> {};
+#ifndef RG_EXACT_ARITH
 template <>
 struct FastMath<double> : NewtonMath {};
+#endif
 
 template <typename T>
 __device__ __forceinline__ T fmax3(T a, T b, T c) {
@@ -451,7 +466,7 @@ __device__ __forceinline__ void wavespeed(const T q[9], const PST<T>& s, const M
   const T f1 = vcon[D] * (T(1) - omsq);
   const T f2 = T(1) - vsq * omsq;
   const T f3 = omsq * (T(1) - vsq) * ((T(1) - vsq * omsq) * gc3dd - (T(1) - omsq) * vcon[D] * vcon[D]);
-  const T sf3 = ma.sqrt(f3), if2 = ma.rcp1(f2);
+  const T sf3 = ma.sqrt(f3), if2 = ma.rcp(f2);
   vfp = (f1 + sf3) * if2;
   vfm = (f1 - sf3) * if2;
   vfp = alpha1 * vfp - betad;
