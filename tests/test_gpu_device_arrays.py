@@ -22,7 +22,8 @@ def test_device_upload_and_download_equal_host(gpu_ctx, kw, offset):
     torch.cuda.synchronize()
     r.step(1)
     r.upload_prims_ptr(buf.data_ptr() + 8 * offset, t0=0.5)
-    out = torch.zeros_like(buf)
+    out = torch.full_like(buf, float("nan"))
+    torch.cuda.synchronize()  # the download runs on the context's stream, which does not wait for torch's
     r.download_prims_ptr(out.data_ptr() + 8 * offset)
     assert np.array_equal(out[offset:].cpu().numpy(), u.ravel())
     r.step(1)
