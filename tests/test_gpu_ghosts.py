@@ -37,3 +37,35 @@ def test_one_pass_equals_the_passes(gpu_ctx, codes, cells):
     got, want = r.bnd_part("bnd4", u, u), o.bnd_part("bnd4", u, u)
     r.release()
     assert np.array_equal(got, want)
+
+
+def test_batched_passes_equal_the_oracle(gpu_ctx):
+    """A batch with a member whose codes need the separate passes (fixed, linear,
+    parabolic and difference-keeping radial ghosts, other codes for other
+    variables): its ghost tiles take one variable each, and the members whose
+    codes one pass could fill take them too.  Against the oracle, step by step,
+    and bit for bit against the same runs alone."""
+    odd = [[5, 4, 3, 5, 5, 2, 7, 2, 4], [2, 18, 18, 4, 3, 5, 7, 5, 2], [1] * 9, [1] * 9,
+           [14, 14, 14, 12, 14, 5, 14, 13, 12], [14, 14, 14, 12, 14, 5, 2, 14, 12]]
+    params = [dict(config.torus(nr=48, nth=40), guard=1, ibc=odd), dict(config.torus(nr=36, nth=44), guard=1)]
+    oracles = [Oracle(p) for p in params]
+    batch, alone = [gpu_ctx.admit(p) for p in params], [gpu_ctx.admit(p) for p in params]
+    for n, o in enumerate(oracles):
+        o.ic_torus(seed=40 + n)
+        o.init_cons()
+        for r in (batch[n], alone[n]):
+            r.upload_prims(o.prims())
+    for _ in range(3):
+        for o in oracles:
+            o.step(1)
+        gpu_ctx.step_batch(batch, 1)
+        for a, b, o in zip(alone, batch, oracles):
+            a.step(1)
+            got, want = b.prims(), o.prims()
+            assert np.array_equal(a.prims(), got)
+            scale = np.maximum(np.abs(want).reshape(-1, 9).max(axis=0), 1e-300)
+            assert (np.abs(got - want).reshape(-1, 9).max(axis=0) / scale).max() < 1e-12  # the per-step parity bound
+            a.upload_prims(want, t0=o.time)
+            b.upload_prims(want, t0=o.time)
+    for r in batch + alone:
+        r.release()
