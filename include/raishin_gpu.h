@@ -158,7 +158,9 @@ int rg_run_ic_torus_device(rg_ctx* ctx, int run, uint64_t seed, double amp, doub
  * rho log-uniform in [0.1, 10], p log-uniform in [0.01, 100], |v| <= 0.9,
  * B^x in [0, 5] shared by both sides, B^y, B^z in [-5, 5].  Sets time = 0. */
 int rg_run_ic_tube(rg_ctx* ctx, int run, uint64_t seed, uint64_t tube);
-/* Host <-> device primitives, layout a(nv,i,j,k).  Upload also sets time = t0. */
+/* Host <-> device primitives, layout a(nv,i,j,k).  Upload also sets time = t0.
+ * The array may be host memory, or device memory whose contents are complete
+ * when the call is made; it has been read, or written, when the call returns. */
 int rg_run_upload_prims(rg_ctx* ctx, int run, const double* uri, double t0);
 int rg_run_download_prims(rg_ctx* ctx, int run, double* uri);
 

@@ -404,8 +404,10 @@ cudaError_t kb_go(const BatchPlan* B, const BLaunch& L, Body body, cudaStream_t 
 
 // Cell kernels run 128-thread blocks (the CT kernel 256) whatever the batch,
 // so a run's cells go through the same compiled code alone and in any mix;
-// MINB keeps each kernel's register budget of the single-run launch (FP64
-// faces 96, FP32 faces 64, update 168 registers).
+// MINB sets each kernel's register budget: that of the single-run launch (FP32
+// faces 64, update 168), but 128 for the FP64 faces (single direct launch 96,
+// where the three directions in one kernel spill 330 B: a 256x256 slab takes
+// 2.48 ms at 96, 2.11 at 128, 2.25 at 168).
 template <int IREC, typename T, typename S>
 cudaError_t go_flux(const BatchPlan* B, const BLaunch& L, cudaStream_t s) {
   const FluxB<IREC, T, S> b{L.stage};

@@ -669,7 +669,13 @@ int drain_events(rg_ctx* ctx) {
   return RG_OK;
 }
 
-// Stored cells below which a stage's three face kernels run side by side.
+// Stored cells up to which a stage's three face kernels run side by side.  What
+// it gains is the gaps between small launches and their last rounds of blocks;
+// beyond, each direction fills the GPU several times over.  FP64 MP5 steps, in turn against
+// side by side: 15,360 cells 0.226 / 0.199 ms, 98,304 0.277 / 0.260, 215,040
+// 0.440 / 0.431, 270,336 0.504 / 0.504, 409,600 0.697 / 0.701, 655,360 0.980 /
+// 0.999.  (The direct and the mixed kernels still gain 2-4% at 650,000; PPM
+// crosses at about 600,000.)
 constexpr long long kForkFaces = 1 << 18;
 
 // One RK3 stage (main.f90:807-911 / 919-1032 / 1043-1147).
@@ -685,9 +691,9 @@ int run_stage(rg_ctx* ctx, Run* R, int stage, const double* Pn, const double* Pc
                                  R->b.F[dir - 1], fs)
                : launch_flux(d, dir, Pc, R->b.F[dir - 1], fs);
   };
-  // The three directions read the same state and write arrays of their own.  On
-  // a grid whose faces of one direction fill the GPU less than about twice
-  // they run side by side (timed runs keep one kernel at a time).
+  // The three directions read the same state and write arrays of their own: on
+  // small grids (3D ones, and slab runs that are not batched) they run side by
+  // side (timed runs keep one kernel at a time).
   const long long nface = (long long)d.imax * d.jpl * d.kpl;
   if (ctx->prof || nface > kForkFaces) {
     RG_CUDA(issue(ctx, K_FLUX1, nf, [&] { return faces(1, s); }));
@@ -833,9 +839,9 @@ struct Snapshot {
   }
 };
 
-// Build and capture the batched step of runs of one class.  A class that
-// has been tuned in this context (e.g. a serving batch whose members changed)
-// gets its tuned shape at once; otherwise the batch starts with the default
+// Build and capture the batched step of runs of one class.  A class and size
+// that has been tuned in this context (e.g. a serving batch whose members
+// changed) gets its tuned shape at once; otherwise the batch starts with the default
 // shape (128-thread blocks, one block per tile, one block per tile along i)
 // and is tuned by tune_batch once it has run kTuneAfter steps, so that the
 // trial steps see the evolved state (shocks, deferred Newton-Raphson cells)
@@ -875,7 +881,7 @@ int make_batch(rg_ctx* ctx, std::vector<Run*>& rs, const std::vector<int>& ids, 
 // that start from a snapshot of the members' current state, restores the
 // state after each, and keeps the fastest.  The shape decides which block
 // computes which cells, never a cell's arithmetic.  The choice is kept per
-// batch class for later batches of the context.
+// batch class and size (tune_class) for later batches of the context.
 int tune_batch(rg_ctx* ctx, BatchEntry* E) {
   cudaStream_t s = ctx->stream;
   std::vector<Run*> rs;

@@ -1346,12 +1346,12 @@ __device__ __forceinline__ void face_thread(const DevRun& r, S* __restrict__ F, 
   }
 }
 
-// Resident blocks of 128 threads per SM the FP64 face kernel is compiled for
-// (registers per thread <= 65536 / (128 * blocks), in steps of 8).
+// Resident blocks of 128 threads per SM the face kernels are compiled for
+// (registers per thread <= 65536 / (128 * blocks), in steps of 8): the direct
+// FP64 kernel; the staged ones in FP64 and FP32.
 #ifndef RG_FLUX_MINB64
 #define RG_FLUX_MINB64 5
 #endif
-
 #ifndef RG_FACE_MINB64
 #define RG_FACE_MINB64 4
 #endif
@@ -1380,26 +1380,35 @@ template <int D, int IREC, typename T, typename S>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? RG_FLUX_MINB64 : 8) k_flux(DevRun r, const S* __restrict__ P, S* __restrict__ F,
                                               float* __restrict__ Fcopy, int icopy, int ilo, int ihi) { flux_body<D, IREC, T, S>(r, P, F, Fcopy, icopy, ilo, ihi, blockIdx); }
 
-// The face kernel (PPM, MP5, WENO5, WENO-Z, WENO-M) with its stencil staged in shared memory by one TMA
-// tile load per block (cp.async.bulk.tensor, this GPU's own buffer, no
-// multicast), in FP64 (S = double) or for the FP32 half of the mixed path
-// (S = float, over P32).  A block takes the same 32 x 2 faces as k_flux (32
-// along i, two rows along j, one k); the tensor map views the primitives as
-// the 4D array (i, j, k, v) and the box covers the block's stencil for all
-// nine variables: 40 x 2 x 1 cells for r faces (i-2 .. i+3 of 32 faces), X x
-// 7 x 1 for phi faces (two rows, j-2 .. j+3 each), X x 2 x 6 for theta faces,
-// with X = 34 (FP64) or 36 (FP32).  The box starts on a 16-byte boundary
-// along i (the TMA's rule): its origin is rounded down to an even (FP64) or
-// a multiple-of-four (FP32) index and the view offsets the lanes by the
-// remainder.  Cells past the array read as zeros (the TMA's out-of-bounds
-// fill); only lanes working on a clamped face could reach them, and those
-// store nothing.  The wait on the transaction barrier is bounded: if the copy
-// has not landed after kTmaWaitCap polls or kTmaWaitNs of the global timer,
-// the block counts C_TMAWAIT, waits once more (bounded) for the copy and
+// The face kernel (PPM, MP5, WENO5, WENO-Z, WENO-M) with its stencil staged in
+// shared memory by TMA tile loads (cp.async.bulk.tensor, this GPU's own buffer,
+// no multicast), in FP64 (S = double) or for the FP32 half of the mixed path
+// (S = float, over P32).  A block of 128 threads takes 32 faces along i in four
+// rows, along j (r and phi faces) or along k (theta faces), one face a thread.
+// The tensor map views the primitives as the 4D array (i, j, k, v); one load
+// brings each of the eight variables that are reconstructed, for MP5 in FP64
+// 38 x 4 x 1 cells for r faces (i-2 .. i+3 of 32 faces), 34 x 9 x 1 for phi faces
+// (four rows, j-2 .. j+3 each) and 34 x 1 x 9 for theta faces; FP64 blocks also
+// load the 16 planes of the face metric that a state reads.  A box starts on a
+// 16-byte boundary along i (the TMA's rule): its origin is rounded down to an
+// even (FP64) or a multiple-of-four (FP32) index and the view offsets the
+// threads by the remainder.  Cells past the array read as zeros (the TMA's
+// out-of-bounds fill); only threads without a face could reach them, and those
+// return.
+//
+// Bound by the fixed latency of dependent FP64 arithmetic (pipe 57-59% busy at
+// 16 warps); in FP32 by issue.  256x128x128 MP5, ms a step and direction: two
+// lanes a face 1.22-1.29, one thread a face with both states in registers (168,
+// 12 warps) 1.12-1.21, with the left state in shared memory, 128 registers and
+// four blocks 0.91-0.98.  (PPM's theta box leaves room for three: 60,416 B.)
+//
+// The wait on the transaction barrier is bounded: if the copies have not landed
+// after kTmaWaitCap polls or kTmaWaitNs of the global timer,
+// the block counts C_TMAWAIT, waits once more (bounded) for the copies and
 // returns without computing; the host reports RG_ECUDA.  A block still
 // waiting after 1024 polls also gives up once the run's count is set, so a
 // launch whose copies never land ends after about one timed-out wave.  (The
-// count is read only there: the normal path issues its copy at once.)
+// count is read only there: the normal path issues its copies at once.)
 constexpr int kTmaWaitCap = 1 << 22;
 constexpr unsigned long long kTmaWaitNs = 50000000ull;  // 50 ms
 
@@ -2375,8 +2384,8 @@ __global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b, si
 // ------------------------------------------------------ scalars of a step
 // The step's loop top (main.f90:617-620): its time, whether it is still
 // taken, and the start of the CFL reduction (cdtcfl.f90:30).  Run where the
-// step before it ends (k_step_end) and where a run's time is set (scal_begin
-// on the host does the same), so that a step opens with the reduction.
+// step before it ends (k_step_end) and where a run's time is set (set_time on
+// the host does the same), so that a step opens with the reduction.
 __device__ __forceinline__ void step_begin_body(const DevRun& r) {
   Scal* s = r.scal;
   if (!s->active) return;
@@ -2881,10 +2890,10 @@ static int fp64_split(const DevRun& r, int lo, int hi) {
   return r.i_fp64 < lo ? lo - 1 : (r.i_fp64 > hi ? hi : r.i_fp64);
 }
 
-// The staged kernel covers the reconstructions whose lanes read their
-// stencil alone, at most two cells either side of the owner cell (the box
-// holds i-2 .. i+3 of its faces): PPM, MP5, WENO5, WENO-Z and WENO-M, whose
-// ghost widths (nm0 = 3, 4) keep the box origin at or above index 0.  MP-WENO
+// The staged kernel covers the reconstructions whose states read their
+// stencil alone, two (PPM: three) cells either side of the owner cell: PPM, MP5,
+// WENO5, WENO-Z and WENO-M, whose ghost widths (nm0 = 3, 4) keep the box origin
+// at or above index 0.  MP-WENO
 // also reads a cell eleven away, the second-order schemes are cheap to read.
 bool flux_tma_eligible(const DevRun& r) {
   const bool scheme = r.irec == 5 || r.irec == 6 || r.irec == 7 || r.irec == 9 || r.irec == 10;

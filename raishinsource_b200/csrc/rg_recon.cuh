@@ -380,6 +380,7 @@ enum PpmCoef {
   PC_X3,     // (x(m) - x(m-1))^3 + (x(m+1) - x(m))^3
   kPpmCoef
 };
+static_assert(kPpmCoef == kPpmPlanes, "one plane of the tables per coefficient");
 
 // interp Eq. (60)-(61) (rec.f90:1346-1418); the theta direction lacks the
 // factor 2 of r and phi (rec.f90:1414).

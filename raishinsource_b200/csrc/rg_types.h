@@ -96,7 +96,7 @@ struct DevRun {
   float* F32[3];         // FP32 face fluxes per direction, 9*N each
   float* CT32;           // FP32 flux-CT values, 6*N
   // PPM's coefficients of the spacings per direction (PpmCoef in rg_recon.cuh,
-  // kPpmCoef planes of n_d values at index m-1; only for irec 5)
+  // kPpmPlanes planes of n_d values at index m-1; only for irec 5)
   const double* ppm[3];
   const float* ppm32[3];  // the same evaluated in FP32 (mixed runs)
   // Limiter coefficients per direction d (MC, minmod, LimO3, MVL, Koren,
