@@ -61,23 +61,20 @@ BYTES_PER_UNIT = {"flux_r": 136, "flux_phi": 136, "flux_theta": 136, "update": 4
                   "floors": 120, "cfl": 72}
 # DRAM bytes per unit measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of one launch divided by
 # its units) on the 192x96x96 torus, whose state already exceeds the L2
-# (update: the TMA-staged k_update_tma, stages 2 and 3, whose boxes re-read their j-1 / k-1 halos)
-DRAM_BYTES_PER_UNIT = {"update": 472.0, "flux_r": 113.0, "flux_phi": 120.0, "flux_theta": 122.0}
+# (update: the TMA-staged k_update_tma, stage 2, whose boxes re-read their j-1 / k-1 halos; faces: k_flux_tma)
+DRAM_BYTES_PER_UNIT = {"update": 587.0, "flux_r": 119.0, "flux_phi": 120.0, "flux_theta": 126.0}
 BYTES_PER_UNIT["flux"] = 136
-# the TMA-staged face kernels (k_flux_tma, stencil and face metric staged) of the FP64 MP5 path, ncu on the
-# 192x96x96 torus
-DRAM_BYTES_PER_UNIT["flux"] = (124.0 + 132.0 + 135.0) / 3
+DRAM_BYTES_PER_UNIT["flux"] = (119.0 + 120.0 + 126.0) / 3
 # FP64 pipe utilisation of the face kernels from ncu (sm__inst_executed_pipe_fp64, percent of the peak
-# sustained rate while active), mean over the three directions (update: over the three stages) on the
-# 192x96x96 torus
-FP64_PIPE_FRAC = {"flux": 0.481, "update": 0.271}
+# sustained rate while active), mean over the three directions (update: stage 2) on the 192x96x96 torus
+FP64_PIPE_FRAC = {"flux": 0.579, "update": 0.273}
 # algorithmic HBM bytes of one zone-update (FP64): only primitives persist between stages
 STEP_BYTES_PER_ZONE = 648
 # Executed FP64 operations per zone-update of one full RK3 step (MP5, FP64): ncu
 # smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum over every launch of one step
 # of the 192x96x96 torus, dadd + dmul + 2 dfma, divided by its interior cells (1,424,896).  It
-# includes the Newton iterations of the FP64 divisions and square roots.
-FP64_FLOPS_PER_ZONE = 15271.0
+# includes the Newton and Goldschmidt iterations of the FP64 divisions and square roots.
+FP64_FLOPS_PER_ZONE = 14795.0
 
 
 def fp64_peak_tflops(device) -> float:
@@ -297,7 +294,7 @@ def run_gpu(args) -> dict | None:
         kinds = {"flux": {"ms": sum(prof[k]["ms"] for k in fam), "launches": sum(prof[k]["launches"] for k in fam)}}
         kinds.update({k: prof[k] for k in prof if k in BYTES_PER_UNIT and k not in fam})
         top = max(kinds, key=lambda k: kinds[k]["ms"])
-        # one update per stage comprises the cell kernel, the straggler pass and the W-carry pass
+        # one update per stage comprises the cell kernel and the straggler and W-carry pass
         n_launch = 3 * args.prof_steps if top == "update" else kinds[top]["launches"]
         nm0, nm1 = run.nm0, run.nm1
         faces = (p["imax"] - 2 * nm0 + 1) * (p["jmax"] - 2 * nm0 + 1) * (p["kmax"] - 2 * nm0 + 1)
@@ -309,13 +306,13 @@ def run_gpu(args) -> dict | None:
         per_launch_ms = kinds[top]["ms"] / max(n_launch, 1)
         achieved = BYTES_PER_UNIT[top] * u / (per_launch_ms * 1e-3) / 1e9
         traffic = DRAM_BYTES_PER_UNIT.get(top)
-        roofline = {"bound": "hbm", "kernel": "k_flux (r, phi, theta faces)" if top == "flux" else top,
+        roofline = {"bound": "hbm", "kernel": "k_flux_tma (r, phi, theta faces)" if top == "flux" else top,
                     "achieved": achieved, "peak": peak, "peak_source": peak_kind,
                     "unit": "GB/s", "frac": achieved / peak,
                     "traffic": None if traffic is None else traffic * u,
                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per unit on the "
                                       "192x96x96 torus, scaled by the units of one launch "
-                                      "(profiles/k_flux_tma_vs_k_flux_fm_torus_3d_192x96x96_mp5.md)",
+                                      "(profiles/k_flux_tma_one_thread_fm_torus_3d_192x96x96_mp5.md)",
                     "bytes_per_unit": BYTES_PER_UNIT[top], "units_per_launch": u, "ms_per_launch": per_launch_ms,
                     "share_of_step": round(kinds[top]["ms"] / total, 4),
                     "fp64_pipe_frac": FP64_PIPE_FRAC.get(top),
