@@ -2192,7 +2192,7 @@ __global__ void k_bc_phys(DevRun r, double* __restrict__ P, const double* __rest
 __device__ __forceinline__ int mirror_src(int code, int n, int L, int nm1, double& sign) {
   if (code == 5) return n <= nm1 ? 1 + nm1 : L - nm1;
   if (code == 13) sign = 0.0;
-  if (code == 12) sign = -sign;
+  if (code == 12) sign = -1.0;
   return n <= nm1 ? 2 * nm1 - n + 1 : 2 * L - 2 * nm1 + 1 - n;
 }
 // The ghost cells, numbered: theta ghosts (whole planes), then phi ghosts of the
@@ -2243,20 +2243,23 @@ __device__ __forceinline__ void bc_all_body(const DevRun& r, double* __restrict_
   double val[9];
 #pragma unroll
   for (int v = 0; v < 9; ++v) {
-    double sign = 1.0;
+    double sr = 1.0, st = 1.0;  // what the r and the theta pass do to the value: keep it, negate it, zero it
     int si = i, sk = k;
-    if (gk) sk = mirror_src(r.ibc[k <= nm1 ? 4 : 5][v], k, r.kmax, nm1, sign);
+    if (gk) sk = mirror_src(r.ibc[k <= nm1 ? 4 : 5][v], k, r.kmax, nm1, st);
     if (gi) {
       const int code = r.ibc[i <= nm1 ? 0 : 1][v];
       if (code == 18) {  // x1 outer (bnd.f90:598-610): zero when u^r of the last interior cell is negative
         si = r.imax - nm1;
-        if (P[N + r.cell(si, sj, sk)] < 0.0) sign = 0.0;
+        if (P[N + r.cell(si, sj, sk)] < 0.0) sr = 0.0;
       } else {
-        si = mirror_src(code, i, r.imax, nm1, sign);
+        si = mirror_src(code, i, r.imax, nm1, sr);
       }
     }
-    const double x = P[(size_t)v * N + r.cell(si, sj, sk)];
-    val[v] = sign == 1.0 ? x : (sign == 0.0 ? 0.0 : -x);
+    double x = P[(size_t)v * N + r.cell(si, sj, sk)];
+    // in the order of the passes: a radial zero negated by the theta pass is -0
+    if (sr != 1.0) x = sr == 0.0 ? 0.0 : -x;
+    if (st != 1.0) x = st == 0.0 ? 0.0 : -x;
+    val[v] = x;
   }
 #pragma unroll
   for (int v = 0; v < 9; ++v) P[(size_t)v * N + c] = val[v];

@@ -39,6 +39,23 @@ def test_one_pass_equals_the_passes(gpu_ctx, codes, cells):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("codes", [
+    _codes([13, 5], [13, 18], [12], [12]),   # a zero of the r pass is negated by the theta pass
+    _codes([12], [14, 18], [13, 12], [12, 5]),
+])
+def test_one_pass_keeps_the_sign_of_zero(gpu_ctx, codes):
+    p = dict(config.torus(nr=20, nth=19, nph=13), guard=1, ibc=codes, flags=config.FLAG_FULL)
+    o = Oracle(p)
+    o.ic_torus(seed=5)
+    u = np.random.default_rng(11).standard_normal(o.prims().shape)
+    u[::3] = 0.0
+    r = gpu_ctx.admit(p)
+    got, want = r.bnd_part("bnd4", u, u), o.bnd_part("bnd4", u, u)
+    r.release()
+    assert (np.signbit(want) & (want == 0)).any()
+    assert np.array_equal(got, want) and np.array_equal(np.signbit(got), np.signbit(want))
+
+
 def test_batched_passes_equal_the_oracle(gpu_ctx):
     """A batch with a member whose codes need the separate passes (fixed, linear,
     parabolic and difference-keeping radial ghosts, other codes for other
